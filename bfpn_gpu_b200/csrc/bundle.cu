@@ -44,7 +44,7 @@ struct Tuning {
     bool tuned = false;
     int tr_ac = 16;       // angles per whole-plane transport block (8 or 16)
     int dst_stages = 2;   // DST ring stages (2 or 3)
-    bool ring = true;     // energy: 4-lane ring kernel (else the 2-lane register kernel)
+    bool ring = true;     // energy: four lanes per thread (else one)
     std::string report;
 };
 
@@ -71,6 +71,7 @@ struct Plan {
     LaunchTable e0a, e0b, e1a, e1b, t0, t1, a0, a1;
     size_t fin = 0;
     int n_fin = 0;
+    int max_ng = 0;  // of the planned slots
 };
 
 }  // namespace
@@ -127,7 +128,9 @@ struct DeviceScope {
 };
 
 // Blocks of one slot entry in each launch.
-int energy_blocks(const bfpn_bundle* b) { return energy_grid(b->lanes, 128); }
+int energy_blocks(const bfpn_bundle* b, bool src, bool dose) {
+    return energy_grid(4, b->lanes, b->NA, src, dose, b->tune.ring ? 4 : 1);
+}
 long long transport_blocks(const bfpn_bundle* b, int Ng) {
     if (b->row_stream) return static_cast<long long>(Ng) * ((b->NA + 7) / 8);
     if (b->cl) return static_cast<long long>(Ng) * ((b->NA + 7) / 8) * b->cl;
@@ -168,13 +171,14 @@ bfpn_status build_plan(bfpn_bundle* b, const std::vector<int>& prim, const std::
     Plan p;
     p.prim = prim;
     p.sec = sec;
-    const long long eb = energy_blocks(b);
+    for (int s : prim) p.max_ng = std::max(p.max_ng, b->slots[s].ctx->Ng);
     auto energy = [&](const std::vector<int>& list, int species, bool src, bool partials) {
         std::vector<EnergyArgs<float>> v;
         for (int s : list) {
             bfpn_ctx* c = b->slots[s].ctx;
             v.push_back(bundle_energy_args(c, species, src, partials ? bundle_partials(c, species) : nullptr));
         }
+        const long long eb = energy_blocks(b, src, partials);
         return add_table(img, v, [&](const EnergyArgs<float>&) { return eb; });
     };
     auto transport = [&](const std::vector<int>& list, int species) {
@@ -210,7 +214,8 @@ bfpn_status build_plan(bfpn_bundle* b, const std::vector<int>& prim, const std::
     std::vector<IddFinalArgs> fin;
     for (int s : prim) {
         const bool has_sec = std::find(sec.begin(), sec.end(), s) != sec.end();
-        fin.push_back(bundle_finalize_args(b->slots[s].ctx, has_sec));
+        fin.push_back(bundle_finalize_args(b->slots[s].ctx, has_sec, energy_blocks(b, false, true),
+                                           energy_blocks(b, true, true)));
     }
     p.fin = img.put(fin);
     p.n_fin = static_cast<int>(fin.size());
@@ -242,9 +247,9 @@ const A* at(const bfpn_bundle* b, size_t off) {
 }
 const int* begin_of(const bfpn_bundle* b, const LaunchTable& t) { return at<int>(b, t.begin); }
 
-cudaError_t enq_energy_t(bfpn_bundle* b, const LaunchTable& t, cudaStream_t s) {
+cudaError_t enq_energy_t(bfpn_bundle* b, const LaunchTable& t, bool src, bool dose, cudaStream_t s) {
     return launch_energy_slots(at<EnergyArgs<float>>(b, t.args), begin_of(b, t), t.n, static_cast<int>(t.work),
-                               b->mode, b->tune.ring, 128, s);
+                               b->mode, b->tune.ring, src, dose, b->plan.max_ng, b->lanes, b->NA, s);
 }
 cudaError_t enq_transport_t(bfpn_bundle* b, const LaunchTable& t, cudaStream_t s) {
     if (b->row_stream)
@@ -278,15 +283,16 @@ cudaError_t enq_bundle_step(bfpn_bundle* b, double* times) {
         times[cls] += ms;
         return r;
     };
-    auto half = [&](const LaunchTable& ea, const LaunchTable& tt, const LaunchTable& aa, const LaunchTable& ebb) {
+    auto half = [&](const LaunchTable& ea, const LaunchTable& tt, const LaunchTable& aa, const LaunchTable& ebb,
+                    bool src) {
         cudaError_t r;
-        if ((r = timed(TK_ENERGY, [&] { return enq_energy_t(b, ea, s); })) != cudaSuccess) return r;
+        if ((r = timed(TK_ENERGY, [&] { return enq_energy_t(b, ea, src, false, s); })) != cudaSuccess) return r;
         if ((r = timed(TK_TRANSPORT, [&] { return enq_transport_t(b, tt, s); })) != cudaSuccess) return r;
         if ((r = timed(TK_ANGLE, [&] { return enq_angle_t(b, aa, s); })) != cudaSuccess) return r;
         if ((r = timed(TK_TRANSPORT, [&] { return enq_transport_t(b, tt, s); })) != cudaSuccess) return r;
-        return timed(TK_ENERGY, [&] { return enq_energy_t(b, ebb, s); });
+        return timed(TK_ENERGY, [&] { return enq_energy_t(b, ebb, src, true, s); });
     };
-    if ((e = half(p.e0a, p.t0, p.a0, p.e0b)) != cudaSuccess) return e;
+    if ((e = half(p.e0a, p.t0, p.a0, p.e0b, false)) != cudaSuccess) return e;
     if (!p.sec.empty()) {
         // each slot's source from its primary, on parallel branches
         const int k = std::min<int>(kMaxSideStreams, static_cast<int>(p.sec.size()));
@@ -299,7 +305,7 @@ cudaError_t enq_bundle_step(bfpn_bundle* b, double* times) {
             if ((e = cudaEventRecord(b->ev_join[i], b->side[i])) != cudaSuccess) return e;
             if ((e = cudaStreamWaitEvent(s, b->ev_join[i], 0)) != cudaSuccess) return e;
         }
-        if ((e = half(p.e1a, p.t1, p.a1, p.e1b)) != cudaSuccess) return e;
+        if ((e = half(p.e1a, p.t1, p.a1, p.e1b, true)) != cudaSuccess) return e;
     }
     return launch_finalize_idd_slots(at<IddFinalArgs>(b, p.fin), p.n_fin, s);
 }
@@ -385,7 +391,7 @@ bfpn_status autotune(bfpn_bundle* b, const std::vector<int>& prim, int max_steps
                       b->key.c_str(),
                       b->row_stream ? "row-streaming" : b->cl ? "cluster" : (best.tr_ac == 16 ? "16 angles/block" : "8 angles/block"),
                       tA[TK_TRANSPORT], tB[TK_TRANSPORT], best.dst_stages, tA[TK_ANGLE], tB[TK_ANGLE],
-                      best.ring ? "4-lane ring" : "2-lane register", tA[TK_ENERGY], tB[TK_ENERGY]);
+                      best.ring ? "4 lanes per thread" : "1 lane per thread", tA[TK_ENERGY], tB[TK_ENERGY]);
         best.report = buf;
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         g_tune[b->key] = best;

@@ -73,19 +73,19 @@ struct Layout {
     int hist_cap;
 };
 
-Layout layout_of(const bfpn_grid& g, int prec, int energy_block) {
+Layout layout_of(const bfpn_grid& g, int prec) {
     Layout L;
     L.per_e = static_cast<long long>(g.Ny + 1) * (g.Nz + 1) * g.Nmu * g.Nom;
     L.cells = L.per_e * g.Ng;
     L.elem = prec == BFPN_PREC_FP64 ? sizeof(double) : sizeof(float);
-    L.part_blocks = std::max({energy_grid(L.per_e, energy_block), idd_partials_grid(L.per_e),
+    L.part_blocks = std::max({energy_grid_most(L.elem, L.per_e, g.Nmu * g.Nom), idd_partials_grid(L.per_e),
                               lite_energy_grid(L.per_e)});
     L.hist_cap = std::max(2 * g.Nx + 16, 4096);
     return L;
 }
 
 uint64_t footprint(const bfpn_grid& g, int prec, bool lite) {
-    const Layout L = layout_of(g, prec, 128);
+    const Layout L = layout_of(g, prec);
     const uint64_t arr = static_cast<uint64_t>(L.cells) * L.elem;
     const uint64_t NA = static_cast<uint64_t>(g.Nmu) * g.Nom;
     uint64_t b = 0;
@@ -359,7 +359,7 @@ cudaError_t enq_energy(bfpn_ctx* c, int species, const double* coef, bool with_s
     a.Ny = c->Ny;
     a.Nz = c->Nz;
     a.trapezoidal = (c->p.flags & BFPN_FLAG_TRAPEZOIDAL_YZ) ? 1 : 0;
-    return prof(c, BFPN_KERNEL_ENERGY, [&] { return launch_energy<T>(a, c->energy_block, c->stream); });
+    return prof(c, BFPN_KERNEL_ENERGY, [&] { return launch_energy<T>(a, c->stream); });
 }
 
 // ng >= 0: the arrays hold ng groups (a chunk of the out-of-core mode).
@@ -552,7 +552,7 @@ cudaError_t enq_primary_half(bfpn_ctx* c, double* partP) {
 
 template <typename T>
 cudaError_t enq_finalize(bfpn_ctx* c, const double* partP, const double* partS, int nS) {
-    const int nP = energy_grid(c->per_e, c->energy_block);
+    const int nP = energy_grid(c->elem, c->per_e, c->NA, false, true);
     const double w = c->d.du * c->d.dv * c->d.dy * c->d.dz;
     return prof(c, BFPN_KERNEL_IDD, [&] {
         return launch_finalize_idd(partP, nP, partS, nS, w, c->d.dg, c->hist_idd, c->hist_proxy, c->counter,
@@ -573,7 +573,7 @@ cudaError_t enq_secondary_half(bfpn_ctx* c, const double* partP, cudaEvent_t pre
     if ((e = enq_energy<T>(c, 1, c->ecoef_half, true, nullptr)) != cudaSuccess) return e;
     if ((e = enq_tat_pair<T>(c, 1, true, true, false, true)) != cudaSuccess) return e;
     if ((e = enq_energy<T>(c, 1, c->ecoef_half, true, partS)) != cudaSuccess) return e;
-    return enq_finalize<T>(c, partP, partS, energy_grid(c->per_e, c->energy_block));
+    return enq_finalize<T>(c, partP, partS, energy_grid(c->elem, c->per_e, c->NA, true, true));
 }
 
 // The IDD of a step without a secondary half (step 0, primary-only and
@@ -653,13 +653,13 @@ cudaError_t enq_overlap_body(bfpn_ctx* c, int step) {
 bool fused_ok(const bfpn_ctx* c) {
     const unsigned fl = c->p.flags;
     if (!c->fuse_energy || !c->overlap || c->prec != BFPN_PREC_MIXED || c->lite || c->ooc ||
-        !transport_in_place(c) || c->energy_block != 128)
+        !transport_in_place(c))
         return false;
     if (fl & (BFPN_FLAG_ENERGY_ONLY | BFPN_FLAG_PRIMARY_ONLY | BFPN_FLAG_NO_TRANSPORT | BFPN_FLAG_NO_ANGLE |
               BFPN_FLAG_LEGACY_ENERGY))
         return false;
     const int mode = (fl & BFPN_FLAG_EQ15_STRAGGLING) ? EMODE_EQ15_STRAG : EMODE_EQ15;
-    if (!energy_fused_supported(c->per_e, mode, c->NA)) return false;
+    if (!energy_fused_supported(mode)) return false;
     // the secondary's source must read the operand the fused kernel writes
     return c->n_groups == 0 || (c->use_umma && c->ablob && c->bblob && c->eblob);
 }
@@ -811,7 +811,7 @@ bfpn_status ensure_ooc(bfpn_ctx* c) {
             else cudaGetLastError();  // without it the source stays on the CUDA-core kernels
         }
     }
-    const size_t part = 4 * static_cast<size_t>(c->n_lc) * energy_grid(c->lc, c->energy_block);
+    const size_t part = 4 * static_cast<size_t>(c->n_lc) * energy_grid_most(c->elem, c->lc, c->NA);
     if ((s = dalloc(c, &c->ooc_part, part * sizeof(double))) != BFPN_OK) return s;
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     c->ooc_ready = true;
@@ -845,7 +845,7 @@ cudaError_t ooc_pass_end(bfpn_ctx* c) {
 // energy_grid(lc) partial pairs per chunk, chunk after chunk (*count in total).
 template <typename T>
 cudaError_t ooc_energy_pass(bfpn_ctx* c, int species, bool with_source, double* partials, int* count) {
-    const int gpc = energy_grid(c->lc, c->energy_block);
+    const int gpc = energy_grid(c->elem, c->lc, c->NA, with_source, true);
     cudaError_t e;
     for (int k = 0; k < c->n_lc; ++k) {
         const int sl = k & 1;
@@ -878,7 +878,7 @@ cudaError_t ooc_energy_pass(bfpn_ctx* c, int species, bool with_source, double* 
         a.Ny = c->Ny;
         a.Nz = c->Nz;
         a.trapezoidal = (c->p.flags & BFPN_FLAG_TRAPEZOIDAL_YZ) ? 1 : 0;
-        if ((e = prof(c, BFPN_KERNEL_ENERGY, [&] { return launch_energy<T>(a, c->energy_block, c->stream); })) !=
+        if ((e = prof(c, BFPN_KERNEL_ENERGY, [&] { return launch_energy<T>(a, c->stream); })) !=
             cudaSuccess)
             return e;
         // out: after the chunk's kernels
@@ -930,7 +930,7 @@ cudaError_t ooc_step(bfpn_ctx* c, bool first, bool secondary_zero) {
     const unsigned fl = c->p.flags;
     const bool energy_only = fl & BFPN_FLAG_ENERGY_ONLY;
     const bool do_tr = !(fl & BFPN_FLAG_NO_TRANSPORT), do_an = !(fl & BFPN_FLAG_NO_ANGLE);
-    const size_t half = 2 * static_cast<size_t>(c->n_lc) * energy_grid(c->lc, c->energy_block);
+    const size_t half = 2 * static_cast<size_t>(c->n_lc) * energy_grid_most(c->elem, c->lc, c->NA);
     double* partP = static_cast<double*>(c->ooc_part);
     double* partS = partP + half;
     int nP = 0, nS = 0;
@@ -1377,7 +1377,7 @@ bfpn_status bfpn_create(const bfpn_grid* grid, const bfpn_phys* phys, int precis
         c->ang_slices = static_cast<int>(std::max<size_t>(1, std::min<size_t>(32, (48 * 1024) / per_slice)));
     }
     const size_t arr = static_cast<size_t>(c->cells) * c->elem;
-    const Layout L = layout_of(*grid, precision, c->energy_block);
+    const Layout L = layout_of(*grid, precision);
     c->n_part = L.part_blocks;
     c->hist_cap = L.hist_cap;
     bfpn_status s;
@@ -2233,13 +2233,12 @@ double* bundle_partials(bfpn_ctx* c, int species) {
     return species == 0 ? primary_partials(c, 0) : c->partials + 2 * static_cast<size_t>(c->n_part);
 }
 
-IddFinalArgs bundle_finalize_args(bfpn_ctx* c, bool secondary) {
+IddFinalArgs bundle_finalize_args(bfpn_ctx* c, bool secondary, int nP, int nS) {
     IddFinalArgs f;
-    const int nP = energy_grid(c->per_e, c->energy_block);
     f.p = bundle_partials(c, 0);
     f.n = nP;
     f.p2 = secondary ? bundle_partials(c, 1) : nullptr;
-    f.n2 = secondary ? nP : 0;
+    f.n2 = secondary ? nS : 0;
     f.idd_scale = c->d.du * c->d.dv * c->d.dy * c->d.dz;
     f.proxy_scale = c->d.dg;
     f.hist_idd = c->hist_idd;

@@ -11,30 +11,23 @@ namespace bfpn {
 // include/config.hpp:38-41 of the reference.
 constexpr double kEpsilon = 1e-10;
 
-// Number of double coefficients per energy group in the energy-sweep table
-// (see tables.cpp: build_energy_coefficients).
-constexpr int kEnergyCoef = 20;
+// Doubles per energy group in the energy-sweep table: eight pairs (psi^1 row,
+// psi^2 row) of the group's linear update (kernels_energy.cu; built by
+// tables.cpp: energy_coefficients).
+constexpr int kEnergyCoef = 16;
 enum EnergyCoef {
-    EC_INV_F = 0,      // 1 / max(1/dt + a_lo/2 + sig/2, eps)
-    EC_A = 1,          // 1.5 a_hi * inv_F
-    EC_F_FROM_F = 2,   // 0.5 a_lo * inv_F
-    EC_F_FROM_HI = 3,  // 0.5 a_hi * inv_F
-    EC_C_UP = 4,       // 0.5 a_hi          (common term: up)
-    EC_C_CUR = 5,      // -0.5 a_lo         (common term: cur)
-    EC_C_F = 6,        // 1/dt - 0.5 sig    (common term: F_g)
-    EC_R_F = 7,        // coefficient of f_g in rhs1e + rhs2e
-    EC_R_UP = 8,       // 1.5 a_hi
-    EC_R_CUR = 9,      // 1.5 a_lo
-    EC_R_FG = 10,      // -1.5 (a_lo + a_hi)
-    EC_R_HI = 11,      // 1.5 a_hi - 0.5 A a_hi
-    EC_INV_COE = 12,   // 1 / max(coe, eps)
-    EC_S_HI = 13,      // straggling: 0.5 rho T_hi / dg2
-    EC_S_LO = 14,      // straggling: 0.5 rho T_lo / dg2
-    EC_S_G = 15,       // straggling: rho T_g / dg2
-    EC_L_IDT = 16,     // legacy: 1/dt
-    EC_L_HI = 17,      // legacy: rho S_hi / dg
-    EC_L_INV_DEN = 18, // legacy: 1 / max(denominator, eps)
-    EC_L_LAP = 19      // legacy straggling: 0.5 dt T_g / dg2 (0 when off)
+    EC_F = 0,    // old psi^1 of the group
+    EC_f = 2,    // old psi^2
+    EC_UP = 4,   // psi^1 - psi^2 of the group above, old
+    EC_D = 6,    // psi^1 - psi^2 of the group above, new
+    EC_SRC = 8,  // source
+    EC_HI = 10,  // straggling: old psi^1 of the group above
+    EC_LO = 12,  // straggling: old psi^1 of the group below
+    // legacy model
+    EC_L_IDT = 0,      // 1/dt
+    EC_L_HI = 1,       // rho S_hi / dg
+    EC_L_INV_DEN = 2,  // 1 / max(denominator, eps)
+    EC_L_LAP = 3       // 0.5 dt T_g / dg2 (0 without straggling)
 };
 
 enum EnergyMode { EMODE_EQ15 = 0, EMODE_EQ15_STRAG = 1, EMODE_LEGACY = 2 };
@@ -69,11 +62,10 @@ __host__ __device__ inline size_t umma_kmajor_offset(int row, int k, int rows) {
 }
 
 // The primary's closing energy half-step of one depth step fused with the
-// opening half-step of the next (no source; float state, lanes a multiple of
-// 4, eq15 modes).  e.F / e.f hold the state after the step's transport and
+// opening half-step of the next (no source; float state, eq15 modes).  e.F / e.f hold the state after the step's transport and
 // angular diffusion and receive the state after the next step's opening
 // half; e.partials receives the closing pass's IDD partials (one pair per
-// block, as energy_ring_kernel).  At the midpoint (after the closing pass)
+// block, as energy_kernel).  At the midpoint (after the closing pass)
 // the state of every source group is also written, split into bf16 hi / lo,
 // as the A operand of the source's angular contraction (rows 0..63 of a
 // 64-position tile max(psi^1, 0), rows 64..127 psi^2, K-major core layout,
@@ -85,7 +77,7 @@ struct EnergyFusedArgs {
     int n_mt, nk;
 };
 cudaError_t launch_energy_fused(const EnergyFusedArgs& a, cudaStream_t s);
-bool energy_fused_supported(long long lanes, int mode, int NA);
+bool energy_fused_supported(int mode);
 
 // Arguments of one transport half-step (Eq. 18) over one array.
 template <typename T>
@@ -169,11 +161,12 @@ struct IddFinalArgs {
 // thread's capture of a larger launch and that graph's replay.
 cudaError_t allow_dynamic_smem(const void* func, size_t need);
 
-// Energy sweep: ring = the 4-lane ring kernel (lanes % 4 == 0, not legacy),
-// else the register kernel with `block` threads; every slot's grid is that
-// kernel's energy_grid of its lanes.
+// Energy sweep: vec = four lanes per thread (NA a multiple of 4), else one;
+// src / dose: whether the slots have a source / sum the dose; max_ng: the
+// slots' largest Ng; every slot's grid is
+// energy_grid(4, lanes, NA, src, dose, vec ? 4 : 1).
 cudaError_t launch_energy_slots(const EnergyArgs<float>* args, const int* begin, int nslots, int blocks, int mode,
-                                bool ring, int block, cudaStream_t s);
+                                bool vec, bool src, bool dose, int max_ng, long long lanes, int NA, cudaStream_t s);
 // Transport of square planes of NP = Ny + 1 points, paired angles: the
 // whole-plane kernel with ang_chunk angles per block (NP a compiled plane
 // size; slot grid Ng * ceil(NA / ang_chunk)) or, for a compiled cluster size,
@@ -197,7 +190,7 @@ int angle_slots_tile(int N);
 cudaError_t launch_finalize_idd_slots(const IddFinalArgs* args, int nslots, cudaStream_t s);
 
 // Launchers (kernels_*.cu).  All return the launch status.
-template <typename T> cudaError_t launch_energy(const EnergyArgs<T>& a, int block, cudaStream_t s);
+template <typename T> cudaError_t launch_energy(const EnergyArgs<T>& a, cudaStream_t s);
 // Lite-memory primary step over psi^1 with fused IDD partials (psi^2 column 0);
 // lc = [Ng][2] (S_hi/dg, max(denom, eps)); lite_energy_grid(lanes) partial pairs.
 template <typename T>
@@ -300,7 +293,20 @@ template <typename T> cudaError_t launch_transport_tiles(const TransportArgs<T>&
 size_t transport_tile_smem(int R, int ac, size_t elem);
 size_t transport_plane_smem(int NP, int ac, size_t elem);
 
-int energy_grid(long long lanes, int block);
+// Blocks of an energy pass over lanes = positions x NA with or without a source
+// and dose sums (one IDD partial pair per block); lanes_per_thread 1 or the
+// vector width (4 float, 2 double), 0: the pass's own choice.  energy_grid_most:
+// the most of any pass.
+int energy_grid(size_t elem, long long lanes, int NA, bool src, bool dose, int lanes_per_thread = 0);
+int energy_grid_most(size_t elem, long long lanes, int NA);
+// The passes whose lanes run in operand tiles: the primary's closing passes,
+// whose IDD partials the fused pass's are.
+__host__ __device__ constexpr bool energy_tiled(bool src, bool dose) { return dose && !src; }
+constexpr int kEnergyMaxLanes = 640;  // lanes of one energy block
+// Shared memory of the staged group constants (pairs each, dose weights with dose).
+__host__ __device__ constexpr size_t energy_table_bytes(int Ng, int pairs, bool dose, bool staged) {
+    return staged ? static_cast<size_t>(Ng) * (pairs + (dose ? 1 : 0)) * 16 : 0;
+}
 int idd_partials_grid(long long lanes);
 
 // Message that bfpn_last_error(NULL) returns on this thread, for entry points

@@ -116,7 +116,6 @@ struct bfpn_ctx {
     bool tr_tile = false;       // use it
     int tr_tile_ac = 8;
     int ang_slices = 4;
-    int energy_block = 128;
 
     cudaGraphExec_t graph_exec = nullptr;
     int graph_key = -1;
@@ -176,9 +175,10 @@ AngleArgs<float> bundle_angle_args(bfpn_ctx* c, int species, int coef, int* err)
 // The secondary source of the context's current primary, enqueued on s.
 cudaError_t bundle_source(bfpn_ctx* c, cudaStream_t s);
 // IDD partial buffers of a step: the primary's and the secondary's, and
-// their counts; the finalisation arguments (secondary = false: the
-// secondary contributes nothing, as on the first step).
-IddFinalArgs bundle_finalize_args(bfpn_ctx* c, bool secondary);
+// their counts nP, nS (energy_grid of the bundle's passes); the finalisation
+// arguments (secondary = false: the secondary contributes nothing, as on the
+// first step).
+IddFinalArgs bundle_finalize_args(bfpn_ctx* c, bool secondary, int nP, int nS);
 double* bundle_partials(bfpn_ctx* c, int species);
 // Room for n more IDD history entries; drops the context's own step graphs.
 bfpn_status bundle_reserve_history(bfpn_ctx* c, int n);

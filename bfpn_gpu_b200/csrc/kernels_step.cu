@@ -1,5 +1,5 @@
-// Depth-step kernels: eq15 energy sweep (with fused IDD partials), MUSCL
-// predictor-corrector transport, separable DST-I angular diffusion, IDD
+// Depth-step kernels: the lite-memory energy step, MUSCL predictor-corrector
+// transport, separable DST-I angular diffusion, IDD
 // finalisation, beam initialisation and conversions.
 //
 // State layout (HBM): index = (ek * nyz + pos) * NA + ang, ang fastest, the
@@ -8,8 +8,6 @@
 
 #include "common.cuh"
 #include "async_copy.cuh"
-
-#include <cuda_bf16.h>
 
 #include <cooperative_groups.h>
 
@@ -50,607 +48,6 @@ cudaError_t allow_dynamic_smem(const void* func, size_t need) {
 
 template <typename T>
 cudaError_t launch_angle_generic(const AngleArgs<T>& a, cudaStream_t s);
-
-// ---------------------------------------------------------------------------
-// Energy sweep (energyDgCnKernel, energy_solver.cu:41-161).
-//
-// One thread per lane (pos, ang); groups are swept from Ng-1 down to 0.  The
-// recursion runs in double for both state types.  The sweep is in place: the
-// old value of group ek+1 (needed by the eq15 "up" term) is kept in a
-// register, the old value of group ek-1 (straggling) is the prefetched load,
-// so no temporaries and no copies back are needed (the reference writes
-// temporaries and copies them back, energy_solver.cu:492-505).
-// Per-group constants come precomputed in a [Ng][kEnergyCoef] table; loads of
-// it are uniform across the warp.
-// When partials != nullptr the kernel also accumulates this species' share of
-// the Eq. 24 depth dose and the psi^2 sum, and writes one pair per block.
-// ---------------------------------------------------------------------------
-constexpr int kEnergyLanesPerThread = 2;
-
-// One group of the eq15 / legacy recursion for one lane (energyDgCnKernel,
-// energy_solver.cu:88-159): Fg, fg old values of group ek, sg its source,
-// Fn the old psi^1 of group ek-1 (straggling), F_hi_old / f_hi_old the old
-// values of group ek+1 and next_F / next_f its new values.
-template <int MODE>
-__device__ __forceinline__ void energy_lane_update(const double* __restrict__ c, int ek, double Fg, double fg,
-                                                   double sg, double Fn, double F_hi_old, double f_hi_old,
-                                                   double next_F, double next_f, double& Fv, double& fv) {
-    if (MODE == EMODE_LEGACY) {
-        const double idt = __ldg(c + EC_L_IDT), hi = __ldg(c + EC_L_HI), inv = __ldg(c + EC_L_INV_DEN);
-        Fv = (fmax(Fg, 0.0) * idt + hi * next_F + sg) * inv;
-        fv = (fg * idt + hi * next_f) * inv;
-        const double lapc = __ldg(c + EC_L_LAP);
-        if (lapc > 0.0) {
-            const double Flo = (ek > 0) ? Fn : 0.0;
-            Fv += lapc * (fmax(F_hi_old, 0.0) - 2.0 * fmax(Fg, 0.0) + fmax(Flo, 0.0));
-        }
-        Fv = fmax(Fv, 0.0);
-        fv = fmax(fv, 0.0);
-    } else {
-        const double up = F_hi_old - f_hi_old;
-        const double cur = Fg - fg;
-        double common = __ldg(c + EC_C_UP) * up + __ldg(c + EC_C_CUR) * cur + __ldg(c + EC_C_F) * Fg + sg;
-        if (MODE == EMODE_EQ15_STRAG) {
-            const double Flo = (ek > 0) ? Fn : 0.0;
-            common += __ldg(c + EC_S_HI) * F_hi_old + __ldg(c + EC_S_LO) * Flo - __ldg(c + EC_S_G) * Fg;
-        }
-        const double hi_delta = next_F - next_f;
-        const double rhs = __ldg(c + EC_R_F) * fg + __ldg(c + EC_R_UP) * up + __ldg(c + EC_R_CUR) * cur +
-                           __ldg(c + EC_R_FG) * Fg - __ldg(c + EC_A) * common + __ldg(c + EC_R_HI) * hi_delta;
-        fv = rhs * __ldg(c + EC_INV_COE);
-        Fv = __ldg(c + EC_F_FROM_F) * fv + __ldg(c + EC_INV_F) * common + __ldg(c + EC_F_FROM_HI) * hi_delta;
-    }
-}
-
-// The sweep of block `bid` of one beam's lanes (the kernels below map their
-// blocks onto it: one beam, or the slots of a bundle).
-// The eq15 constants of one group held in registers (loaded a group ahead by
-// the ring sweep, so their loads are off the recursion's critical path), and
-// the eq15 update of energy_lane_update from them: the same operations in the
-// same order.
-struct Eq15Coef {
-    double c_up, c_cur, c_f, r_f, r_up, r_cur, r_fg, a, r_hi, inv_coe, f_from_f, inv_f, f_from_hi;
-    double s_hi, s_lo, s_g;  // straggling
-    double d0, d1;           // dose weights of psi^1, psi^2
-};
-
-template <int MODE>
-__device__ __forceinline__ Eq15Coef load_eq15_coef(const double* __restrict__ c, const double* __restrict__ dc,
-                                                   bool dose) {
-    Eq15Coef k;
-    k.c_up = __ldg(c + EC_C_UP);
-    k.c_cur = __ldg(c + EC_C_CUR);
-    k.c_f = __ldg(c + EC_C_F);
-    k.r_f = __ldg(c + EC_R_F);
-    k.r_up = __ldg(c + EC_R_UP);
-    k.r_cur = __ldg(c + EC_R_CUR);
-    k.r_fg = __ldg(c + EC_R_FG);
-    k.a = __ldg(c + EC_A);
-    k.r_hi = __ldg(c + EC_R_HI);
-    k.inv_coe = __ldg(c + EC_INV_COE);
-    k.f_from_f = __ldg(c + EC_F_FROM_F);
-    k.inv_f = __ldg(c + EC_INV_F);
-    k.f_from_hi = __ldg(c + EC_F_FROM_HI);
-    k.s_hi = k.s_lo = k.s_g = 0.0;
-    if (MODE == EMODE_EQ15_STRAG) {
-        k.s_hi = __ldg(c + EC_S_HI);
-        k.s_lo = __ldg(c + EC_S_LO);
-        k.s_g = __ldg(c + EC_S_G);
-    }
-    k.d0 = dose ? __ldg(dc) : 0.0;
-    k.d1 = dose ? __ldg(dc + 1) : 0.0;
-    return k;
-}
-
-template <int MODE>
-__device__ __forceinline__ void eq15_update(const Eq15Coef& k, int ek, double Fg, double fg, double sg, double Fn,
-                                            double F_hi_old, double f_hi_old, double next_F, double next_f,
-                                            double& Fv, double& fv) {
-    const double up = F_hi_old - f_hi_old;
-    const double cur = Fg - fg;
-    double common = k.c_up * up + k.c_cur * cur + k.c_f * Fg + sg;
-    if (MODE == EMODE_EQ15_STRAG) {
-        const double Flo = (ek > 0) ? Fn : 0.0;
-        common += k.s_hi * F_hi_old + k.s_lo * Flo - k.s_g * Fg;
-    }
-    const double hi_delta = next_F - next_f;
-    const double rhs = k.r_f * fg + k.r_up * up + k.r_cur * cur + k.r_fg * Fg - k.a * common + k.r_hi * hi_delta;
-    fv = rhs * k.inv_coe;
-    Fv = k.f_from_f * fv + k.inv_f * common + k.f_from_hi * hi_delta;
-}
-
-template <int MODE, typename T, int LPT, int D>
-__device__ __forceinline__ void energy_body(const EnergyArgs<T>& a, long long bid) {
-    // D: groups prefetched ahead of use
-    const long long L = a.lanes;
-    const int Ng = a.Ng;
-    long long lane[LPT];
-    bool ok[LPT];
-#pragma unroll
-    for (int j = 0; j < LPT; ++j) {
-        lane[j] = bid * blockDim.x * LPT + threadIdx.x + j * blockDim.x;
-        ok[j] = lane[j] < L;
-    }
-    const T* __restrict__ sp = a.src;
-    // ring of the next D groups' old values for each lane
-    T rF[D][LPT], rf[D][LPT], rs[D][LPT];
-#pragma unroll
-    for (int k = 0; k < D; ++k)
-#pragma unroll
-        for (int j = 0; j < LPT; ++j) {
-            const int e = Ng - 1 - k;
-            const bool in = ok[j] && e >= 0;
-            rF[k][j] = in ? a.F[e * L + lane[j]] : T(0);
-            rf[k][j] = in ? a.f[e * L + lane[j]] : T(0);
-            rs[k][j] = (in && sp) ? sp[e * L + lane[j]] : T(0);
-        }
-    double F_hi_old[LPT], f_hi_old[LPT], next_F[LPT], next_f[LPT], w_pos[LPT], acc = 0.0, accp = 0.0;
-#pragma unroll
-    for (int j = 0; j < LPT; ++j) {
-        F_hi_old[j] = f_hi_old[j] = next_F[j] = next_f[j] = 0.0;
-        w_pos[j] = 1.0;
-        if (a.partials && a.trapezoidal && ok[j]) {
-            const int pos = static_cast<int>((lane[j] + a.lane0) / a.NA);
-            const int iy = pos % (a.Ny + 1), iz = pos / (a.Ny + 1);
-            if (iy == 0 || iy == a.Ny) w_pos[j] *= 0.5;
-            if (iz == 0 || iz == a.Nz) w_pos[j] *= 0.5;
-        }
-    }
-    for (int base = Ng - 1; base >= 0; base -= D)
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-        const int ek = base - k;
-        if (ek < 0) break;
-        const double* __restrict__ c = a.coef + ek * kEnergyCoef;
-        const double* __restrict__ dc = a.dose_coef + 2 * ek;
-        const int ep = ek - D;  // the group that refills this slot
-#pragma unroll
-        for (int j = 0; j < LPT; ++j) {
-            const double Fg = static_cast<double>(rF[k][j]), fg = static_cast<double>(rf[k][j]),
-                         sg = static_cast<double>(rs[k][j]);
-            if (ep >= 0 && ok[j]) {
-                rF[k][j] = a.F[ep * L + lane[j]];
-                rf[k][j] = a.f[ep * L + lane[j]];
-                if (sp) rs[k][j] = sp[ep * L + lane[j]];
-            }
-            // old value of group ek-1 (straggling): the next slot, or the refill of slot 0
-            const double Fn = static_cast<double>(rF[(k + 1) % D][j]);
-            double Fv, fv;
-            energy_lane_update<MODE>(c, ek, Fg, fg, sg, Fn, F_hi_old[j], f_hi_old[j], next_F[j], next_f[j], Fv, fv);
-            const T Fs = static_cast<T>(Fv), fs = static_cast<T>(fv);
-            if (ok[j]) {
-                a.F[ek * L + lane[j]] = Fs;
-                a.f[ek * L + lane[j]] = fs;
-                if (a.partials) {
-                    acc += w_pos[j] * (__ldg(dc) * static_cast<double>(Fs) + __ldg(dc + 1) * static_cast<double>(fs));
-                    accp += static_cast<double>(fs);
-                }
-            }
-            F_hi_old[j] = Fg;
-            f_hi_old[j] = fg;
-            next_F[j] = Fv;
-            next_f[j] = fv;
-        }
-    }
-    if (a.partials) {
-        __shared__ double red[2][32];
-        for (int o = 16; o > 0; o >>= 1) {
-            acc += __shfl_down_sync(0xffffffffu, acc, o);
-            accp += __shfl_down_sync(0xffffffffu, accp, o);
-        }
-        const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-        if (l == 0) {
-            red[0][w] = acc;
-            red[1][w] = accp;
-        }
-        __syncthreads();
-        if (w == 0) {
-            const int nw = blockDim.x >> 5;
-            acc = (l < nw) ? red[0][l] : 0.0;
-            accp = (l < nw) ? red[1][l] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) {
-                acc += __shfl_down_sync(0xffffffffu, acc, o);
-                accp += __shfl_down_sync(0xffffffffu, accp, o);
-            }
-            if (l == 0) {
-                a.partials[2 * bid] = acc;
-                a.partials[2 * bid + 1] = accp;
-            }
-        }
-    }
-}
-
-template <int MODE, typename T, int LPT, int D = 4, int NTH = 128, int MINB = (sizeof(T) == 4 ? 5 : 4)>
-__global__ void __launch_bounds__(NTH, MINB) energy_kernel(EnergyArgs<T> a) {
-    energy_body<MODE, T, LPT, D>(a, blockIdx.x);
-}
-
-template <int MODE, int LPT, int D = 4, int NTH = 128, int MINB = 5>
-__global__ void __launch_bounds__(NTH, MINB) energy_slots_kernel(const EnergyArgs<float>* __restrict__ args,
-                                                                  const int* __restrict__ begin, int nslots) {
-    const int s = find_slot(begin, nslots, blockIdx.x);
-    energy_body<MODE, float, LPT, D>(args[s], blockIdx.x - __ldg(begin + s));
-}
-
-// Float state, lanes a multiple of 4: each thread sweeps 4 consecutive lanes
-// and keeps its own ring of the next groups' old values in shared memory,
-// filled by 16-byte cp.async copies (no registers held by the prefetch, no
-// block barrier: a thread only reads what it copied).  Slot i % D holds group
-// Ng-1-i; the slot consumed in one iteration is refilled in the next, so up
-// to D-2 groups are in flight ahead of the one in use.  Same update and IDD
-// partials as energy_kernel.
-constexpr int kEnergyRing = 8, kEnergyRingThreads = 64;
-
-template <int MODE, int D, int NTH>
-__device__ __forceinline__ void energy_ring_body(const EnergyArgs<float>& a, long long bid) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float4* ring = reinterpret_cast<float4*>(smem_raw);  // [D][3][NTH]
-    const long long L = a.lanes;
-    const int Ng = a.Ng, tid = threadIdx.x;
-    const long long lane0 = (bid * NTH + tid) * 4;
-    const bool ok = lane0 < L;  // L % 4 == 0: the 4 lanes are all in or all out
-    const float* __restrict__ sp = a.src;
-    auto slot = [&](int k, int arr) { return ring + (k * 3 + arr) * NTH + tid; };
-    auto fill = [&](int i) {  // group Ng-1-i into slot i % D, one commit group per call
-        const int e = Ng - 1 - i;
-        if (ok && e >= 0) {
-            const size_t off = static_cast<size_t>(e) * L + lane0;
-            cp_async16(slot(i % D, 0), a.F + off, true);
-            cp_async16(slot(i % D, 1), a.f + off, true);
-            if (sp) cp_async16(slot(i % D, 2), sp + off, true);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    for (int i = 0; i < D; ++i) fill(i);
-    double F_hi_old[4], f_hi_old[4], next_F[4], next_f[4], w_pos[4], acc = 0.0, accp = 0.0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        F_hi_old[j] = f_hi_old[j] = next_F[j] = next_f[j] = 0.0;
-        w_pos[j] = 1.0;
-        if (a.partials && a.trapezoidal && ok) {
-            const int pos = static_cast<int>((lane0 + j + a.lane0) / a.NA);
-            const int iy = pos % (a.Ny + 1), iz = pos / (a.Ny + 1);
-            if (iy == 0 || iy == a.Ny) w_pos[j] *= 0.5;
-            if (iz == 0 || iz == a.Nz) w_pos[j] *= 0.5;
-        }
-    }
-    constexpr bool kStrag = MODE == EMODE_EQ15_STRAG;
-    const bool dose = a.partials != nullptr;
-    // group Ng-1-i's constants in K[i % 2]; iteration i loads the next
-    // group's into the other slot.  Two iterations per trip keep the slots
-    // fixed registers instead of a copy of the set per group.
-    Eq15Coef K[2];
-    K[0] = load_eq15_coef<MODE>(a.coef + (Ng - 1) * kEnergyCoef, a.dose_coef + 2 * (Ng - 1), dose);
-    auto iter = [&](auto Rc, int i) {
-        constexpr int R = decltype(Rc)::value;
-        const int ek = Ng - 1 - i;
-        if (ek < 0) return;
-        const Eq15Coef& kc = K[R];
-        if (ek > 0) K[R ^ 1] = load_eq15_coef<MODE>(a.coef + (ek - 1) * kEnergyCoef, a.dose_coef + 2 * (ek - 1), dose);
-        // groups 0 .. i (and i+1 for straggling) have landed
-        if (kStrag) asm volatile("cp.async.wait_group %0;" ::"n"(D - 3) : "memory");
-        else asm volatile("cp.async.wait_group %0;" ::"n"(D - 2) : "memory");
-        const float4 vF = *slot(i % D, 0), vf = *slot(i % D, 1);
-        const float4 vs = sp ? *slot(i % D, 2) : make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 vn = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (kStrag && ek > 0) vn = *slot((i + 1) % D, 0);
-        if (i > 0) fill(i - 1 + D);  // the slot read in the previous iteration
-        const float Fa[4] = {vF.x, vF.y, vF.z, vF.w}, fa[4] = {vf.x, vf.y, vf.z, vf.w};
-        const float sa[4] = {vs.x, vs.y, vs.z, vs.w}, na[4] = {vn.x, vn.y, vn.z, vn.w};
-        float Fo[4], fo[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const double Fg = Fa[j], fg = fa[j];
-            double Fv, fv;
-            eq15_update<MODE>(kc, ek, Fg, fg, static_cast<double>(sa[j]), static_cast<double>(na[j]), F_hi_old[j],
-                              f_hi_old[j], next_F[j], next_f[j], Fv, fv);
-            Fo[j] = static_cast<float>(Fv);
-            fo[j] = static_cast<float>(fv);
-            if (dose && ok) {
-                acc += w_pos[j] * (kc.d0 * static_cast<double>(Fo[j]) + kc.d1 * static_cast<double>(fo[j]));
-                accp += static_cast<double>(fo[j]);
-            }
-            F_hi_old[j] = Fg;
-            f_hi_old[j] = fg;
-            next_F[j] = Fv;
-            next_f[j] = fv;
-        }
-        if (ok) {
-            const size_t off = static_cast<size_t>(ek) * L + lane0;
-            *reinterpret_cast<float4*>(a.F + off) = make_float4(Fo[0], Fo[1], Fo[2], Fo[3]);
-            *reinterpret_cast<float4*>(a.f + off) = make_float4(fo[0], fo[1], fo[2], fo[3]);
-        }
-    };
-#pragma unroll 1
-    for (int i = 0; i < Ng; i += 2) {
-        iter(IntC<0>(), i);
-        iter(IntC<1>(), i + 1);
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (a.partials) {
-        __shared__ double red[2][NTH / 32];
-        for (int o = 16; o > 0; o >>= 1) {
-            acc += __shfl_down_sync(0xffffffffu, acc, o);
-            accp += __shfl_down_sync(0xffffffffu, accp, o);
-        }
-        const int w = tid >> 5, l = tid & 31;
-        if (l == 0) {
-            red[0][w] = acc;
-            red[1][w] = accp;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double s0 = 0.0, s1 = 0.0;
-            for (int k = 0; k < NTH / 32; ++k) {
-                s0 += red[0][k];
-                s1 += red[1][k];
-            }
-            a.partials[2 * bid] = s0;
-            a.partials[2 * bid + 1] = s1;
-        }
-    }
-}
-
-template <int MODE, int D, int NTH>
-__global__ void __launch_bounds__(NTH) energy_ring_kernel(EnergyArgs<float> a) {
-    energy_ring_body<MODE, D, NTH>(a, blockIdx.x);
-}
-
-template <int MODE, int D, int NTH>
-__global__ void __launch_bounds__(NTH) energy_ring_slots_kernel(const EnergyArgs<float>* __restrict__ args,
-                                                                const int* __restrict__ begin, int nslots) {
-    const int s = find_slot(begin, nslots, blockIdx.x);
-    energy_ring_body<MODE, D, NTH>(args[s], blockIdx.x - __ldg(begin + s));
-}
-
-int energy_ring_grid(long long lanes) {
-    const long long per_block = 4LL * kEnergyRingThreads;
-    return static_cast<int>((lanes + per_block - 1) / per_block);
-}
-
-cudaError_t launch_energy_ring(const EnergyArgs<float>& a, cudaStream_t s) {
-    if (a.lanes % 4 != 0 || a.mode == EMODE_LEGACY) return cudaErrorNotSupported;
-    constexpr int D = kEnergyRing, NTH = kEnergyRingThreads;
-    const size_t smem = static_cast<size_t>(D) * 3 * NTH * sizeof(float4);
-    const int grid = energy_ring_grid(a.lanes);
-    if (a.mode == EMODE_EQ15) energy_ring_kernel<EMODE_EQ15, D, NTH><<<grid, NTH, smem, s>>>(a);
-    else energy_ring_kernel<EMODE_EQ15_STRAG, D, NTH><<<grid, NTH, smem, s>>>(a);
-    return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// Fused primary energy half-steps: the closing E1/2 of step n and the opening
-// E1/2 of step n+1 in one sweep over the groups (high -> low).  The opening
-// sweep's update of group g needs the closing result of groups g and g-1
-// (straggling) and its own results for g+1, so it runs one group behind the
-// closing sweep, its carried values in registers: iteration i applies the
-// closing update to group ek = Ng-1-i and the opening update to group ek+1.
-// Each update is energy_ring_kernel's, on the same inputs -- the midpoint
-// value is rounded to float as the separate passes store it -- so the state
-// equals the two passes' bit for bit on the grids tested, except a few values
-// far below the peak, which may come out one float rounding step apart (on a
-// 35 x 35, 12-group grid: values 1e-8 below the peak, 4.6e-16 of it).  The closing pass's IDD partials are those of the
-// closing ring pass.  At the midpoint the source groups' values
-// go to the angular contraction's operand (split bf16), which removes that
-// operand's own pass over the primary.
-// ---------------------------------------------------------------------------
-template <int MODE, int D, int NTH>
-__global__ void __launch_bounds__(NTH) energy_fused_kernel(EnergyFusedArgs A) {
-    const EnergyArgs<float>& a = A.e;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float4* ring = reinterpret_cast<float4*>(smem_raw);  // [D][2][NTH]
-    const long long L = a.lanes;
-    const int Ng = a.Ng, tid = threadIdx.x;
-    const long long bid = blockIdx.x;
-    const long long lane0 = (bid * NTH + tid) * 4;
-    const bool ok = lane0 < L;  // L % 4 == 0: the 4 lanes are all in or all out
-    auto slot = [&](int k, int arr) { return ring + (k * 2 + arr) * NTH + tid; };
-    auto fill = [&](int i) {  // group Ng-1-i into slot i % D, one commit group per call
-        const int e = Ng - 1 - i;
-        if (ok && e >= 0) {
-            const size_t off = static_cast<size_t>(e) * L + lane0;
-            cp_async16(slot(i % D, 0), a.F + off, true);
-            cp_async16(slot(i % D, 1), a.f + off, true);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    for (int i = 0; i < D; ++i) fill(i);
-    // closing sweep: old values and new values of the group above; opening
-    // sweep: midpoint values and new values of the group above its own
-    double cFo[4], cfo[4], cFn[4], cfn[4], oFo[4], ofo[4], oFn[4], ofn[4], w_pos[4], acc = 0.0, accp = 0.0;
-    float mF[4], mf[4];  // midpoint of group ek+1
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        cFo[j] = cfo[j] = cFn[j] = cfn[j] = oFo[j] = ofo[j] = oFn[j] = ofn[j] = 0.0;
-        mF[j] = mf[j] = 0.f;
-        w_pos[j] = 1.0;
-        if (a.partials && a.trapezoidal && ok) {
-            const int pos = static_cast<int>((lane0 + j) / a.NA);
-            const int iy = pos % (a.Ny + 1), iz = pos / (a.Ny + 1);
-            if (iy == 0 || iy == a.Ny) w_pos[j] *= 0.5;
-            if (iz == 0 || iz == a.Nz) w_pos[j] *= 0.5;
-        }
-    }
-    // this thread's place in the source operand: position p, angles k0 .. k0+3 of chunk kc
-    const int p = ok ? static_cast<int>(lane0 / a.NA) : 0, k0 = ok ? static_cast<int>(lane0 % a.NA) : 0;
-    constexpr size_t kPart = 128 * 16 * 2;  // one (hi or lo) 128 x 16 bf16 tile
-    const size_t a_tile = (static_cast<size_t>(p >> 6) * A.nk + (k0 >> 4)) * 2 * kPart;
-    const size_t a_off1 = umma_kmajor_offset(p & 63, k0 & 15, 128), a_off2 = umma_kmajor_offset(64 + (p & 63), k0 & 15, 128);
-    const size_t a_group = static_cast<size_t>(A.n_mt) * A.nk * 2 * kPart;
-    auto put = [&](size_t off, float x0, float x1, float x2, float x3) {  // 4 values: hi, then lo
-        const __nv_bfloat162 h01 = __floats2bfloat162_rn(x0, x1), h23 = __floats2bfloat162_rn(x2, x3);
-        const __nv_bfloat162 l01 = __floats2bfloat162_rn(x0 - __low2float(h01), x1 - __high2float(h01));
-        const __nv_bfloat162 l23 = __floats2bfloat162_rn(x2 - __low2float(h23), x3 - __high2float(h23));
-        uint2 hv, lv;
-        hv.x = *reinterpret_cast<const uint32_t*>(&h01);
-        hv.y = *reinterpret_cast<const uint32_t*>(&h23);
-        lv.x = *reinterpret_cast<const uint32_t*>(&l01);
-        lv.y = *reinterpret_cast<const uint32_t*>(&l23);
-        *reinterpret_cast<uint2*>(A.ablob + off) = hv;
-        *reinterpret_cast<uint2*>(A.ablob + off + kPart) = lv;
-    };
-    constexpr bool kStrag = MODE == EMODE_EQ15_STRAG;
-    const bool dose = a.partials != nullptr;
-    Eq15Coef k_next = load_eq15_coef<MODE>(a.coef + (Ng - 1) * kEnergyCoef, a.dose_coef + 2 * (Ng - 1), dose);
-    Eq15Coef k_up = k_next;  // constants of group ek+1 (the opening update's group)
-    for (int i = 0; i <= Ng; ++i) {
-        const int ek = Ng - 1 - i;
-        float nF[4] = {0.f, 0.f, 0.f, 0.f}, nf[4] = {0.f, 0.f, 0.f, 0.f};  // midpoint of group ek
-        Eq15Coef kc = k_up;
-        if (ek >= 0) {
-            // closing update of group ek
-            kc = k_next;
-            if (ek > 0) k_next = load_eq15_coef<MODE>(a.coef + (ek - 1) * kEnergyCoef, a.dose_coef + 2 * (ek - 1), dose);
-            if (kStrag) asm volatile("cp.async.wait_group %0;" ::"n"(D - 3) : "memory");
-            else asm volatile("cp.async.wait_group %0;" ::"n"(D - 2) : "memory");
-            const float4 vF = *slot(i % D, 0), vf = *slot(i % D, 1);
-            float4 vn = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (kStrag && ek > 0) vn = *slot((i + 1) % D, 0);
-            if (i > 0) fill(i - 1 + D);  // the slot read in the previous iteration
-            const float Fa[4] = {vF.x, vF.y, vF.z, vF.w}, fa[4] = {vf.x, vf.y, vf.z, vf.w};
-            const float na[4] = {vn.x, vn.y, vn.z, vn.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const double Fg = Fa[j], fg = fa[j];
-                double Fv, fv;
-                eq15_update<MODE>(kc, ek, Fg, fg, 0.0, static_cast<double>(na[j]), cFo[j], cfo[j], cFn[j], cfn[j],
-                                  Fv, fv);
-                nF[j] = static_cast<float>(Fv);
-                nf[j] = static_cast<float>(fv);
-                if (dose && ok) {
-                    acc += w_pos[j] * (kc.d0 * static_cast<double>(nF[j]) + kc.d1 * static_cast<double>(nf[j]));
-                    accp += static_cast<double>(nf[j]);
-                }
-                cFo[j] = Fg;
-                cfo[j] = fg;
-                cFn[j] = Fv;
-                cfn[j] = fv;
-            }
-            const int gz = A.ablob ? __ldg(A.gmap + ek) : -1;
-            if (ok && gz >= 0) {
-                const size_t base = static_cast<size_t>(gz) * a_group + a_tile;
-                put(base + a_off1, fmaxf(nF[0], 0.f), fmaxf(nF[1], 0.f), fmaxf(nF[2], 0.f), fmaxf(nF[3], 0.f));
-                put(base + a_off2, nf[0], nf[1], nf[2], nf[3]);
-            }
-        }
-        if (ek + 1 <= Ng - 1) {
-            // opening update of group ek+1 from the midpoint: its value mF/mf,
-            // group ek's (straggling) nF, the group above's oFo/oFn
-            const int eo = ek + 1;
-            float Fo[4], fo[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const double Fg = mF[j], fg = mf[j];
-                double Fv, fv;
-                eq15_update<MODE>(k_up, eo, Fg, fg, 0.0, static_cast<double>(nF[j]), oFo[j], ofo[j], oFn[j], ofn[j],
-                                  Fv, fv);
-                Fo[j] = static_cast<float>(Fv);
-                fo[j] = static_cast<float>(fv);
-                oFo[j] = Fg;
-                ofo[j] = fg;
-                oFn[j] = Fv;
-                ofn[j] = fv;
-            }
-            if (ok) {
-                const size_t off = static_cast<size_t>(eo) * L + lane0;
-                *reinterpret_cast<float4*>(a.F + off) = make_float4(Fo[0], Fo[1], Fo[2], Fo[3]);
-                *reinterpret_cast<float4*>(a.f + off) = make_float4(fo[0], fo[1], fo[2], fo[3]);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            mF[j] = nF[j];
-            mf[j] = nf[j];
-        }
-        k_up = kc;
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (a.partials) {
-        __shared__ double red[2][NTH / 32];
-        for (int o = 16; o > 0; o >>= 1) {
-            acc += __shfl_down_sync(0xffffffffu, acc, o);
-            accp += __shfl_down_sync(0xffffffffu, accp, o);
-        }
-        const int w = tid >> 5, l = tid & 31;
-        if (l == 0) {
-            red[0][w] = acc;
-            red[1][w] = accp;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double s0 = 0.0, s1 = 0.0;
-            for (int k = 0; k < NTH / 32; ++k) {
-                s0 += red[0][k];
-                s1 += red[1][k];
-            }
-            a.partials[2 * bid] = s0;
-            a.partials[2 * bid + 1] = s1;
-        }
-    }
-}
-
-bool energy_fused_supported(long long lanes, int mode, int NA) {
-    return lanes % 4 == 0 && NA % 4 == 0 && mode != EMODE_LEGACY;
-}
-
-cudaError_t launch_energy_fused(const EnergyFusedArgs& A, cudaStream_t s) {
-    const EnergyArgs<float>& a = A.e;
-    if (!energy_fused_supported(a.lanes, a.mode, a.NA) || a.src || a.lane0 != 0) return cudaErrorNotSupported;
-    constexpr int D = kEnergyRing, NTH = kEnergyRingThreads;
-    const size_t smem = static_cast<size_t>(D) * 2 * NTH * sizeof(float4);
-    const int grid = energy_ring_grid(a.lanes);
-    if (a.mode == EMODE_EQ15) energy_fused_kernel<EMODE_EQ15, D, NTH><<<grid, NTH, smem, s>>>(A);
-    else energy_fused_kernel<EMODE_EQ15_STRAG, D, NTH><<<grid, NTH, smem, s>>>(A);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_energy_slots(const EnergyArgs<float>* args, const int* begin, int nslots, int blocks, int mode,
-                                bool ring, int block, cudaStream_t s) {
-    if (nslots <= 0 || blocks <= 0) return cudaSuccess;
-    if (ring) {
-        if (mode == EMODE_LEGACY) return cudaErrorNotSupported;
-        constexpr int D = kEnergyRing, NTH = kEnergyRingThreads;
-        const size_t smem = static_cast<size_t>(D) * 3 * NTH * sizeof(float4);
-        if (mode == EMODE_EQ15) energy_ring_slots_kernel<EMODE_EQ15, D, NTH><<<blocks, NTH, smem, s>>>(args, begin, nslots);
-        else energy_ring_slots_kernel<EMODE_EQ15_STRAG, D, NTH><<<blocks, NTH, smem, s>>>(args, begin, nslots);
-        return cudaGetLastError();
-    }
-    if (block != 128) return cudaErrorNotSupported;
-    constexpr int LPT = kEnergyLanesPerThread;
-    switch (mode) {
-        case EMODE_EQ15: energy_slots_kernel<EMODE_EQ15, LPT><<<blocks, 128, 0, s>>>(args, begin, nslots); break;
-        case EMODE_EQ15_STRAG:
-            energy_slots_kernel<EMODE_EQ15_STRAG, LPT><<<blocks, 128, 0, s>>>(args, begin, nslots);
-            break;
-        default: energy_slots_kernel<EMODE_LEGACY, LPT><<<blocks, 128, 0, s>>>(args, begin, nslots); break;
-    }
-    return cudaGetLastError();
-}
-
-int energy_grid(long long lanes, int block) {
-    const long long per_block = static_cast<long long>(block) * kEnergyLanesPerThread;
-    return static_cast<int>((lanes + per_block - 1) / per_block);
-}
-
-template <typename T>
-cudaError_t launch_energy(const EnergyArgs<T>& a, int block, cudaStream_t s) {
-    constexpr int LPT = kEnergyLanesPerThread;
-    if constexpr (sizeof(T) == 4) {
-        // planes of at least 2^20 lanes fill the GPU with 64-thread ring blocks
-        // (4 lanes a thread); smaller ones keep more threads per SM with the
-        // register ring.  Same partial count: 4 * 64 lanes per block = 2 * 128.
-        if (a.lanes >= (1LL << 20) && a.lanes % 4 == 0 && a.mode != EMODE_LEGACY &&
-            block * LPT == 4 * kEnergyRingThreads)
-            return launch_energy_ring(a, s);
-    }
-    const int grid = energy_grid(a.lanes, block);
-    switch (a.mode) {
-        case EMODE_EQ15: energy_kernel<EMODE_EQ15, T, LPT><<<grid, block, 0, s>>>(a); break;
-        case EMODE_EQ15_STRAG: energy_kernel<EMODE_EQ15_STRAG, T, LPT><<<grid, block, 0, s>>>(a); break;
-        default: energy_kernel<EMODE_LEGACY, T, LPT><<<grid, block, 0, s>>>(a); break;
-    }
-    return cudaGetLastError();
-}
 
 // ---------------------------------------------------------------------------
 // Lite-memory primary step (litePrimaryEnergyStepKernel, bfpm_solver.cu:593-620):
@@ -3106,7 +2503,6 @@ cudaError_t launch_convert(const Tin* in, Tout* out, long long n, cudaStream_t s
 }
 
 #define BFPN_INSTANTIATE(T)                                                                                       \
-    template cudaError_t launch_energy<T>(const EnergyArgs<T>&, int, cudaStream_t);                               \
     template cudaError_t launch_lite_energy<T>(T*, const double*, double, int, long long, const double*, int, int,  \
                                                int, int, double*, cudaStream_t);                                  \
     template cudaError_t launch_transport<T>(const TransportArgs<T>&, int, cudaStream_t);                         \

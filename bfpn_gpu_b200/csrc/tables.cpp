@@ -438,32 +438,42 @@ std::vector<double> energy_coefficients(const BeamTables& t, const bfpn_phys& p,
         const double sig = std::max(t.sigma[ek], 0.0);
         const double S_lo = std::max(t.S_s[ek], 0.0), S_hi = std::max(t.S_s[ek + 1], 0.0);
         const double a_lo = rho * S_lo / dg, a_hi = rho * S_hi / dg;
-        const double inv_F = 1.0 / std::max(idt + 0.5 * a_lo + 0.5 * sig, kEpsilon);
-        const double A = 1.5 * a_hi * inv_F;
-        k[EC_INV_F] = inv_F;
-        k[EC_A] = A;
-        k[EC_F_FROM_F] = 0.5 * a_lo * inv_F;
-        k[EC_F_FROM_HI] = 0.5 * a_hi * inv_F;
-        k[EC_C_UP] = 0.5 * a_hi;
-        k[EC_C_CUR] = -0.5 * a_lo;
-        k[EC_C_F] = idt - 0.5 * sig;
-        k[EC_R_F] = idt - 0.5 * sig - 0.5 * (a_hi - a_lo);
-        k[EC_R_UP] = 1.5 * a_hi;
-        k[EC_R_CUR] = 1.5 * a_lo;
-        k[EC_R_FG] = -1.5 * (a_lo + a_hi);
-        k[EC_R_HI] = 1.5 * a_hi - A * 0.5 * a_hi;
-        const double coe = idt + 0.5 * sig + 1.5 * a_lo + 0.5 * (a_hi - a_lo) + A * 0.5 * a_lo;
-        k[EC_INV_COE] = 1.0 / std::max(coe, kEpsilon);
         const double T_g = strag ? std::max(t.T_c[ek], 0.0) : 0.0;
         const double T_hi = (strag && ek + 1 < Ng) ? std::max(t.T_c[ek + 1], 0.0) : 0.0;
         const double T_lo = (strag && ek > 0) ? std::max(t.T_c[ek - 1], 0.0) : 0.0;
-        k[EC_S_HI] = 0.5 * rho * T_hi / dg2;
-        k[EC_S_LO] = 0.5 * rho * T_lo / dg2;
-        k[EC_S_G] = rho * T_g / dg2;
-        k[EC_L_IDT] = idt;
-        k[EC_L_HI] = a_hi;
-        k[EC_L_INV_DEN] = 1.0 / std::max(idt + a_lo + sig, kEpsilon);
-        k[EC_L_LAP] = T_g > 0.0 ? 0.5 * dt * T_g / dg2 : 0.0;
+        if (p.flags & BFPN_FLAG_LEGACY_ENERGY) {
+            k[EC_L_IDT] = idt;
+            k[EC_L_HI] = a_hi;
+            k[EC_L_INV_DEN] = 1.0 / std::max(idt + a_lo + sig, kEpsilon);
+            k[EC_L_LAP] = T_g > 0.0 ? 0.5 * dt * T_g / dg2 : 0.0;
+            continue;
+        }
+        // energy_solver.cu:108-159 with u = psi^1 - psi^2 of the group above
+        // (old), d the same of its new values and
+        //   common = a_hi/2 u - a_lo/2 (F - f) + (1/dt - sig/2) F + straggling + s
+        // as f' = (rhs1e + rhs2e - A common + r_d d) / coe and
+        // F' = a_lo/2 f'/den + common/den + a_hi/2 d/den, each as its
+        // coefficients of F, f, u, d, s and the straggling neighbours.  Formed
+        // in long double: where sig is far above the other terms the sums
+        // cancel, and a coefficient rounded before that would carry the error.
+        using L = long double;
+        const L lo = L(rho) * S_lo / dg, hi = L(rho) * S_hi / dg, it = L(1) / dt, sg = sig;
+        const L inv_F = L(1) / std::max<L>(it + lo / 2 + sg / 2, kEpsilon), A = L(1.5) * hi * inv_F;
+        const L inv_coe = L(1) / std::max<L>(it + sg / 2 + L(1.5) * lo + (hi - lo) / 2 + A * lo / 2, kEpsilon);
+        const L F_from_f = lo / 2 * inv_F, c_F = it - sg / 2 - lo / 2 - L(rho) * T_g / dg2;
+        const L c_hi = L(rho) * T_hi / dg2 / 2, c_lo = L(rho) * T_lo / dg2 / 2;
+        auto row = [&](int at, L rhs, L common, L direct) {
+            const L f_row = inv_coe * (rhs - A * common);
+            k[at + 1] = static_cast<double>(f_row);
+            k[at] = static_cast<double>(F_from_f * f_row + inv_F * common + direct);
+        };
+        row(EC_F, L(-1.5) * hi, c_F, 0);
+        row(EC_f, it - sg / 2 - (hi - lo) / 2 - L(1.5) * lo, lo / 2, 0);
+        row(EC_UP, L(1.5) * hi, hi / 2, 0);
+        row(EC_D, L(1.5) * hi - A * hi / 2, 0, hi / 2 * inv_F);
+        row(EC_SRC, 0, 1, 0);
+        row(EC_HI, 0, c_hi, 0);
+        row(EC_LO, 0, c_lo, 0);
     }
     return c;
 }
