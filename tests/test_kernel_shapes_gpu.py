@@ -1,0 +1,70 @@
+"""The kernels at the sizes where their tiling can go wrong -- remainders of
+lanes, groups, positions and angles, the smallest and largest of each form --
+against the FP64 oracle.
+
+Tolerances: FP64 operators 1e-11 of the peak, FP64 lite steps 1e-10 (as in
+test_parity_gpu.py).  Float state starts from float values, so an operator's
+error is that of its float arithmetic: one rounding of the result for the
+energy sweep (2^-24 = 6e-8, bar 1e-6), some thirty operations on differences of
+neighbours for the transport (bar 2e-6), four passes of up to 32 products for
+the angular step (4 * 32 * 2^-24 = 8e-6, bar 2e-5)."""
+import numpy as np
+import pytest
+
+from conftest import rel_err
+from test_parity_gpu import OP_TOL, STEP_TOL, assert_states, build, seeded_states, set_both, small_cfg
+from bfpn_gpu_b200 import capi
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+PRECISIONS = [capi.PREC_FP64, capi.PREC_MIXED]
+
+
+def _states(ctx, seed, precision):
+    s = seeded_states(ctx, seed)
+    return [a.astype(np.float32).astype(np.float64) for a in s] if precision == capi.PREC_MIXED else s
+
+
+# (ny, nz, nmu, nom, ng): one lane per thread with 1, 2, 4 and 3 mod 4 groups;
+# vectors (75,776 float / 37,888 double lanes and more) with odd and even groups,
+# whole and partial operand tiles of positions and angles
+ENERGY_SHAPES = [(3, 2, 3, 3, 5), (4, 4, 5, 7, 2), (6, 5, 4, 5, 40), (2, 8, 9, 1, 43), (17, 17, 16, 16, 7),
+                 (20, 21, 14, 14, 6)]
+
+
+def _energy_cfg(shape, **flags):
+    ny, nz, nmu, nom, ng = shape
+    return small_cfg(ny=ny, nz=nz, nmu=nmu, nom=nom, ng=ng, lg=1.475 * ng, beam_energy=1.0 * ng, **flags)
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("flags", [{}, {"eq15_straggling": True, "trapezoidal_yz": True}, {"legacy_energy": True}])
+@pytest.mark.parametrize("shape", ENERGY_SHAPES)
+def test_energy_sweep_shapes(shape, flags, precision):
+    cfg = _energy_cfg(shape, **flags)
+    ctx, ora = build(cfg, precision=precision)
+    set_both(ctx, ora, _states(ctx, 41, precision))
+    ctx.energy(0, 0.5 * cfg.dt())
+    ora.energy(0, 0.5 * cfg.dt())
+    assert_states(ctx, ora, OP_TOL if precision == capi.PREC_FP64 else 1e-6, ((0, 0), (0, 1)))
+
+
+@pytest.mark.parametrize("straggling", [False, True])
+@pytest.mark.parametrize("shape", ENERGY_SHAPES)
+def test_fused_pass_shapes(shape, straggling):
+    """Steps with the fused primary pass against the separate passes, states
+    as test_parity_gpu.py compares them (one rounding far below the peak)."""
+    cfg = _energy_cfg(shape, eq15_straggling=straggling, trapezoidal_yz=straggling)
+    got = []
+    for fused in (0, 1):
+        ctx, _ = build(cfg, precision=capi.PREC_MIXED)
+        ctx.set_option(capi.OPT_STEP_OVERLAP, 2 * fused)
+        ctx.set_option(capi.OPT_FUSED_ENERGY, fused)
+        ctx.step(4)
+        got.append([ctx.get_state(sp, cf) for sp in (0, 1) for cf in (0, 1)])
+    for a, b in zip(*got):
+        peak = np.abs(a).max()
+        assert np.abs(a - b).max() <= 1e-12 * peak
+        big = np.abs(a) >= 1e-6 * peak
+        assert np.array_equal(a[big], b[big])
