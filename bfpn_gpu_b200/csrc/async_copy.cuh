@@ -87,6 +87,13 @@ __device__ __forceinline__ void cp_async_ca(void* dst, const void* src) {
     else
         asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
 }
+// A 16-byte copy under a predicate (no branch, nothing written when off).
+__device__ __forceinline__ void cp_async16_if(void* dst, const void* src, bool on) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(static_cast<int>(on))
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }

@@ -88,7 +88,7 @@ struct bfpn_bundle {
     bool shaped = false;
     std::string key;
     int NP = 0, N = 0, NA = 0, mode = EMODE_EQ15, cl = 0;
-    bool row_stream = false;  // row-streaming transport (else cl > 0: cluster, else whole-plane)
+    int march = 0;  // lines per chunk of the marching transport (else cl > 0: cluster, else whole-plane)
     long long lanes = 0;
     bool no_clip = false;
     Tuning tune;
@@ -132,7 +132,7 @@ int energy_blocks(const bfpn_bundle* b, bool src, bool dose) {
     return energy_grid(4, b->lanes, b->NA, src, dose, b->tune.ring ? 4 : 1);
 }
 long long transport_blocks(const bfpn_bundle* b, int Ng) {
-    if (b->row_stream) return static_cast<long long>(Ng) * ((b->NA + 7) / 8);
+    if (b->march) return static_cast<long long>(Ng) * transport_march_chunks(b->NA, 4);
     if (b->cl) return static_cast<long long>(Ng) * ((b->NA + 7) / 8) * b->cl;
     return static_cast<long long>(Ng) * ((b->NA + b->tune.tr_ac - 1) / b->tune.tr_ac);
 }
@@ -252,9 +252,9 @@ cudaError_t enq_energy_t(bfpn_bundle* b, const LaunchTable& t, bool src, bool do
                                b->mode, b->tune.ring, src, dose, b->plan.max_ng, b->lanes, b->NA, s);
 }
 cudaError_t enq_transport_t(bfpn_bundle* b, const LaunchTable& t, cudaStream_t s) {
-    if (b->row_stream)
-        return launch_transport_stream_slots(at<TransportArgs<float>>(b, t.args), begin_of(b, t), t.n,
-                                             static_cast<int>(t.work), b->NP - 1, b->NA, s);
+    if (b->march)
+        return launch_transport_march_slots(at<TransportArgs<float>>(b, t.args), begin_of(b, t), t.n,
+                                            static_cast<int>(t.work), b->NP - 1, b->NA, b->march, s);
     return launch_transport_slots(at<TransportArgs<float>>(b, t.args), begin_of(b, t), t.n, static_cast<int>(t.work),
                                   b->NP, b->NA, b->tune.tr_ac, b->cl > 0, s);
 }
@@ -379,7 +379,7 @@ bfpn_status autotune(bfpn_bundle* b, const std::vector<int>& prim, int max_steps
     }
     Tuning best = A;
     if (rounds >= 2) {
-        const bool fixed_tr = b->cl || b->row_stream;  // one transport form: nothing to choose
+        const bool fixed_tr = b->cl || b->march;  // one transport form: nothing to choose
         best.tr_ac = (fixed_tr || tA[TK_TRANSPORT] <= tB[TK_TRANSPORT]) ? A.tr_ac : B.tr_ac;
         best.dst_stages = tA[TK_ANGLE] <= tB[TK_ANGLE] ? A.dst_stages : B.dst_stages;
         best.ring = tA[TK_ENERGY] <= tB[TK_ENERGY] ? A.ring : B.ring;
@@ -389,7 +389,7 @@ bfpn_status autotune(bfpn_bundle* b, const std::vector<int>& prim, int max_steps
                       "%s: transport %s (%.3f ms vs %.3f ms per step-pair), DST %d stages (%.3f vs %.3f), "
                       "energy %s (%.3f vs %.3f)",
                       b->key.c_str(),
-                      b->row_stream ? "row-streaming" : b->cl ? "cluster" : (best.tr_ac == 16 ? "16 angles/block" : "8 angles/block"),
+                      b->march ? "marching" : b->cl ? "cluster" : (best.tr_ac == 16 ? "16 angles/block" : "8 angles/block"),
                       tA[TK_TRANSPORT], tB[TK_TRANSPORT], best.dst_stages, tA[TK_ANGLE], tB[TK_ANGLE],
                       best.ring ? "4 lanes per thread" : "1 lane per thread", tA[TK_ENERGY], tB[TK_ENERGY]);
         best.report = buf;
@@ -544,7 +544,7 @@ bfpn_status bfpn_bundle_admit(bfpn_bundle* b, const bfpn_beam* beam, int32_t* sl
         b->mode = mode;
         b->no_clip = no_clip;
         b->cl = bundle_cluster_size(c);
-        b->row_stream = bundle_stream_transport(c);
+        b->march = bundle_march_lines(c);
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         auto it = g_tune.find(key);
         if (it != g_tune.end()) b->tune = it->second;

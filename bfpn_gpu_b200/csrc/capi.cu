@@ -292,21 +292,33 @@ void choose_plane_transport(bfpn_ctx* c) {
     c->tr_stream_ok = c->elem == 4 && transport_stream_supported(c->Ny, c->NA);
 }
 
-// The row-streaming kernel runs this context's transport (it needs paired angles).
+// The marching kernel runs this context's transport: planes without a
+// whole-plane kernel (or any supported one, option 2), in both precisions and
+// for any directions, unless an option names another kernel for the plane.
+bool march_transport(const bfpn_ctx* c) {
+    if (!c->tr_pairs || c->tr_stream == 0 || !transport_march_supported(c->Ny)) return false;
+    if (c->tr_stream == 2) return c->tr_stream_ok && c->tr_pairs_ok;
+    if (c->tr_plane) return false;
+    return (c->tr_stream_ok && c->tr_pairs_ok) || !c->tr_named;
+}
+
+// The row-streaming kernel runs this context's transport (it needs paired
+// angles): planes wider than the marching kernel takes.
 bool stream_transport(const bfpn_ctx* c) {
+    if (march_transport(c)) return false;
     if (!c->tr_stream_ok || !c->tr_pairs || !c->tr_pairs_ok) return false;
     return c->tr_stream == 2 || (c->tr_stream == 1 && !c->tr_plane);
 }
 
 // The cluster kernel runs this context's transport (it needs paired angles).
 bool cluster_transport(const bfpn_ctx* c) {
-    if (stream_transport(c)) return false;
+    if (march_transport(c) || stream_transport(c)) return false;
     if (!c->tr_cluster_ok || !c->tr_pairs || !c->tr_pairs_ok) return false;
     return c->tr_cluster == 2 || (c->tr_cluster == 1 && !c->tr_plane);
 }
 
 bool transport_in_place(const bfpn_ctx* c) {
-    return c->tr_plane || c->tr_inplace || cluster_transport(c) || stream_transport(c);
+    return c->tr_plane || c->tr_inplace || cluster_transport(c) || stream_transport(c) || march_transport(c);
 }
 
 template <typename T>
@@ -380,6 +392,8 @@ cudaError_t enq_transport(bfpn_ctx* c, const void* in, void* out, double dt, boo
     a.tile_z = c->tr_tz;
     a.preserve_sign = preserve_sign ? 1 : 0;
     a.pairs = (c->elem == 4 && c->tr_pairs && c->tr_pairs_ok) ? 1 : 0;
+    if (march_transport(c))
+        return prof(c, BFPN_KERNEL_TRANSPORT, [&] { return launch_transport_march<T>(a, c->tr_lines, c->stream); });
     if constexpr (sizeof(T) == 4) {
         if (stream_transport(c))
             return prof(c, BFPN_KERNEL_TRANSPORT, [&] { return launch_transport_stream(a, c->stream); });
@@ -1503,6 +1517,7 @@ bfpn_status bfpn_load_tables(bfpn_ctx* c, const double* mu, int32_t mu_rows, con
     if ((s = upload_f64(c, c->lite_coef, lite.data(), lite.size() * sizeof(double))) != BFPN_OK) return s;
     if ((s = upload_state_table(c, c->omega, T.omega)) != BFPN_OK) return s;
     c->tr_pairs_ok = transport_pairs_ok(T.omega.data(), c->NA);
+    c->tr_lines = transport_march_lines(T.omega.data(), c->NA, c->elem);
     if ((s = upload_state_table(c, c->fac_step, angle_factor(T, c->p, c->d.dt))) != BFPN_OK) return s;
     if ((s = upload_state_table(c, c->sine_u, T.sine_u)) != BFPN_OK) return s;
     if ((s = upload_state_table(c, c->sine_v, T.sine_v)) != BFPN_OK) return s;
@@ -1858,6 +1873,7 @@ bfpn_status bfpn_set_option(bfpn_ctx* c, int32_t option, int32_t value) {
                 c->tr_tile = value != 0;
                 if (value > 1) c->tr_tile_ac = value;
             }
+            c->tr_named = value != 1;
             break;
         }
         default:
@@ -2155,8 +2171,8 @@ std::string bundle_ready(const bfpn_ctx* c) {
         return "a bundle runs the eq15 step with transport, angular diffusion and secondaries";
     if (!c->tables_loaded || !c->beam_ready) return "load the tables and the initial beam first";
     if (!(c->tr_pairs && c->tr_pairs_ok)) return "the angle pairs do not share direction signs";
-    if (!(stream_transport(c) || cluster_transport(c) || c->tr_plane))
-        return "no whole-plane, row-streaming or cluster transport kernel for this plane";
+    if (!(march_transport(c) || cluster_transport(c) || c->tr_plane))
+        return "no whole-plane, marching or cluster transport kernel for this plane";
     if (c->Nom != c->Nmu || c->Nom % 2 != 0 || c->Nom < 4 || c->Nom > 32 || c->Nom == 26 || c->Nom == 30)
         return "the angular grid must be square with an even side in 4..24, 28 or 32";
     if (c->nyz < angle_slots_tile(c->Nom)) return "the plane is smaller than one DST tile";
@@ -2252,12 +2268,12 @@ bfpn_status bundle_reserve_history(bfpn_ctx* c, int n) { return ensure_history(c
 
 int bundle_cluster_size(const bfpn_ctx* c) { return cluster_transport(c) ? transport_cluster_size(c->Ny + 1) : 0; }
 
-bool bundle_stream_transport(const bfpn_ctx* c) { return stream_transport(c); }
+int bundle_march_lines(const bfpn_ctx* c) { return march_transport(c) ? c->tr_lines : 0; }
 
 std::string bundle_class_key(const bfpn_ctx* c) {
     char buf[160];
     std::snprintf(buf, sizeof buf, "plane %dx%d angles %dx%d %s %s", c->Ny + 1, c->Nz + 1, c->Nmu, c->Nom,
-                  stream_transport(c) ? "row-streaming" : cluster_transport(c) ? "cluster" : "whole-plane",
+                  march_transport(c) ? "marching" : cluster_transport(c) ? "cluster" : "whole-plane",
                   (c->p.flags & BFPN_FLAG_EQ15_STRAGGLING) ? "eq15+straggling" : "eq15");
     return buf;
 }

@@ -178,9 +178,6 @@ int transport_cluster_size(int NP);
 // one block per (group, 8-angle chunk) plane walking the z rows, in place.
 cudaError_t launch_transport_stream(const TransportArgs<float>& a, cudaStream_t s);
 bool transport_stream_supported(int Ny, int NA);
-// The same over the slots of a bundle (slot grid Ng * ceil(NA / 8)).
-cudaError_t launch_transport_stream_slots(const TransportArgs<float>* args, const int* begin, int nslots, int blocks,
-                                          int Ny, int NA, cudaStream_t s);
 // Pipelined paired DST (Nom = Nmu = N even): work tiles of 2 * 128 / N slices;
 // tile_begin = tile offsets (slot s has ceil(Ng nyz / tile) tiles); stages 2 or 3.
 cudaError_t launch_angle_slots(const AngleArgs<float>* args, const int* tile_begin, int nslots, long long tiles,
@@ -287,6 +284,15 @@ bool transport_pairs_ok(const double* omega, int NA);
 // 8-angle chunk) plane, in place.
 cudaError_t launch_transport_cluster(const TransportArgs<float>& a, cudaStream_t s);
 bool transport_cluster_supported(int Ny, int Nz);
+// Marching transport (kernels_march.cu): planes of up to 128 x any points, any
+// directions, in place; lines = transport_march_lines of the omega table
+// ([NA][2]), blocks = Ng * transport_march_chunks.
+template <typename T> cudaError_t launch_transport_march(const TransportArgs<T>& a, int lines, cudaStream_t s);
+cudaError_t launch_transport_march_slots(const TransportArgs<float>* args, const int* begin, int nslots, int blocks,
+                                         int Ny, int NA, int lines, cudaStream_t s);
+bool transport_march_supported(int Ny);
+int transport_march_chunks(int NA, size_t elem);
+int transport_march_lines(const double* omega, int NA, size_t elem);
 // Any plane, in 27 x 27 output tiles with a 4-cell halo, out of place;
 // ang_chunk 4 or 8 (float), 2 or 4 (double).
 template <typename T> cudaError_t launch_transport_tiles(const TransportArgs<T>& a, int ang_chunk, cudaStream_t s);

@@ -115,6 +115,8 @@ struct bfpn_ctx {
     bool tr_tile_ok = false;    // the plane needs tiles: the unrolled tiled kernel applies
     bool tr_tile = false;       // use it
     int tr_tile_ac = 8;
+    bool tr_named = false;      // BFPN_OPT_PLANE_TRANSPORT names the line walks or an angle chunk
+    int tr_lines = 0;           // most lines of any angle chunk of the marching transport
     int ang_slices = 4;
 
     cudaGraphExec_t graph_exec = nullptr;
@@ -187,7 +189,7 @@ bfpn_status bundle_reserve_history(bfpn_ctx* c, int n);
 std::string bundle_class_key(const bfpn_ctx* c);
 // CTAs per cluster of the context's cluster transport, 0 for whole-plane transport.
 int bundle_cluster_size(const bfpn_ctx* c);
-// The context's transport runs the row-streaming kernel.
-bool bundle_stream_transport(const bfpn_ctx* c);
+// Lines per angle chunk of the context's marching transport, 0 where another kernel runs it.
+int bundle_march_lines(const bfpn_ctx* c);
 
 }  // namespace bfpn

@@ -1183,13 +1183,6 @@ __global__ void __maxnreg__(kStreamMaxReg) transport_stream_kernel(TransportArgs
     transport_stream_body(a, n_chunks, blockIdx.x);
 }
 
-__global__ void __maxnreg__(kStreamMaxReg) transport_stream_slots_kernel(const TransportArgs<float>* __restrict__ args,
-                                                                      const int* __restrict__ begin, int nslots,
-                                                                      int n_chunks) {
-    const int s = find_slot(begin, nslots, blockIdx.x);
-    transport_stream_body(args[s], n_chunks, blockIdx.x - __ldg(begin + s));
-}
-
 int transport_stream_threads(int Ny) { return (Ny + 1) * kStreamTPC; }
 
 bool transport_stream_supported(int Ny, int NA) {
@@ -1206,18 +1199,6 @@ cudaError_t launch_transport_stream(const TransportArgs<float>& a, cudaStream_t 
     const long long blocks = static_cast<long long>(a.Ng) * n_chunks;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     transport_stream_kernel<<<static_cast<unsigned>(blocks), transport_stream_threads(a.Ny), smem, s>>>(a, n_chunks);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_transport_stream_slots(const TransportArgs<float>* args, const int* begin, int nslots, int blocks,
-                                          int Ny, int NA, cudaStream_t s) {
-    if (nslots <= 0 || blocks <= 0) return cudaSuccess;
-    if (!transport_stream_supported(Ny, NA)) return cudaErrorNotSupported;
-    const int n_chunks = (NA + 2 * kStreamPairs - 1) / (2 * kStreamPairs);
-    const size_t smem = transport_stream_smem(Ny + 1);
-    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(transport_stream_slots_kernel), smem);
-    if (e != cudaSuccess) return e;
-    transport_stream_slots_kernel<<<blocks, transport_stream_threads(Ny), smem, s>>>(args, begin, nslots, n_chunks);
     return cudaGetLastError();
 }
 

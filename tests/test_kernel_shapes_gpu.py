@@ -68,3 +68,28 @@ def test_fused_pass_shapes(shape, straggling):
         assert np.abs(a - b).max() <= 1e-12 * peak
         big = np.abs(a) >= 1e-6 * peak
         assert np.array_equal(a[big], b[big])
+
+
+# widths: one position to 128 over every (lanes, positions per lane) form and
+# both of its ends; angle grids whose pairs all share signs (4 x 4), partly do
+# (5 x 6, lone angles and mixed warps) or lack a partner (5 x 3, odd rows)
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("ny,nz,ang", [(1, 3, (4, 4)), (2, 1, (5, 6)), (7, 9, (5, 3)), (8, 3, (4, 4)), (11, 2, (5, 6)),
+                                       (23, 5, (5, 3)), (32, 4, (5, 6)), (37, 29, (4, 4)), (47, 2, (2, 2)),
+                                       (48, 5, (5, 6)), (64, 3, (5, 3)), (80, 6, (5, 6)), (95, 2, (4, 4)),
+                                       (96, 3, (5, 6)), (127, 2, (5, 3))])
+def test_march_transport_shapes(ny, nz, ang, precision):
+    cfg = small_cfg(ny=ny, nz=nz, nmu=ang[0], nom=ang[1], ng=3, ly=0.2 * ny, lz=0.25 * nz)
+    ctx, ora = build(cfg, precision=precision)
+    Ng, nyz, NA = ctx.shape
+    states = [a.reshape(Ng, nyz, NA) for a in _states(ctx, 42, precision)]
+    for a in states:
+        a[1, : nyz // 2] = a[1, 0]                                   # flat
+        a[2] = np.float32(3e-11) * np.arange(nyz)[:, None]            # differences around the limiter's epsilon
+    if precision == capi.PREC_MIXED:
+        states = [a.astype(np.float32).astype(np.float64) for a in states]
+    set_both(ctx, ora, [a.ravel() for a in states])
+    for sp, cf, dtf, keep in ((0, 0, 0.5, False), (0, 1, 0.5, True), (1, 0, 0.31, False), (1, 1, 0.5, True)):
+        ctx.transport(sp, cf, dtf * cfg.dt(), keep)
+        ora.transport(sp, cf, dtf * cfg.dt(), keep)
+    assert_states(ctx, ora, OP_TOL if precision == capi.PREC_FP64 else 2e-6)
