@@ -196,6 +196,8 @@ cudaError_t launch_lite_energy(T* F, const double* lc, double dt, int Ng, long l
 int lite_energy_grid(long long lanes);
 template <typename T> cudaError_t launch_transport(const TransportArgs<T>& a, int ang_chunk, cudaStream_t s);
 template <typename T> cudaError_t launch_angle(const AngleArgs<T>& a, cudaStream_t s);
+// Any angular grid up to 32 x 32 (kernels_dst.cu).
+template <typename T> cudaError_t launch_angle_rect(const AngleArgs<T>& a, cudaStream_t s);
 template <typename T> cudaError_t launch_source_angular(const SourceArgs<T>& a, cudaStream_t s);
 template <typename T> cudaError_t launch_source_energy(const SourceArgs<T>& a, int tile_e, cudaStream_t s);
 template <typename T> cudaError_t launch_init_beam(T* F, const double* yza, const double* e, long long per_e,

@@ -93,3 +93,17 @@ def test_march_transport_shapes(ny, nz, ang, precision):
         ctx.transport(sp, cf, dtf * cfg.dt(), keep)
         ora.transport(sp, cf, dtf * cfg.dt(), keep)
     assert_states(ctx, ora, OP_TOL if precision == capi.PREC_FP64 else 2e-6)
+
+
+# rows and columns of different lengths, lengths without a square kernel, one
+# line, odd counts of lines, tiles over the end of a group
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("nom,nmu", [(15, 12), (12, 15), (1, 7), (8, 1), (32, 3), (5, 32), (31, 31), (26, 30), (9, 17)])
+def test_rectangular_angle_shapes(nom, nmu, precision):
+    cfg = small_cfg(ny=4, nz=6, nmu=nmu, nom=nom, ng=5, lz=2.0)
+    ctx, ora = build(cfg, precision=precision)
+    set_both(ctx, ora, _states(ctx, 43, precision))
+    for sp, cf in ((0, 0), (1, 1)):
+        ctx.angle(sp, cf, 0.7 * cfg.dt())
+        ora.angle(sp, cf, 0.7 * cfg.dt())
+    assert_states(ctx, ora, OP_TOL if precision == capi.PREC_FP64 else 2e-5)
