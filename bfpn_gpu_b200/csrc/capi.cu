@@ -78,8 +78,7 @@ Layout layout_of(const bfpn_grid& g, int prec) {
     L.per_e = static_cast<long long>(g.Ny + 1) * (g.Nz + 1) * g.Nmu * g.Nom;
     L.cells = L.per_e * g.Ng;
     L.elem = prec == BFPN_PREC_FP64 ? sizeof(double) : sizeof(float);
-    L.part_blocks = std::max({energy_grid_most(L.elem, L.per_e, g.Nmu * g.Nom), idd_partials_grid(L.per_e),
-                              lite_energy_grid(L.per_e)});
+    L.part_blocks = std::max({energy_grid_most(L.elem, L.per_e, g.Nmu * g.Nom), idd_partials_grid(L.per_e)});
     L.hist_cap = std::max(2 * g.Nx + 16, 4096);
     return L;
 }
@@ -506,12 +505,19 @@ cudaError_t enq_tat(bfpn_ctx* c, int species, int coef, bool do_tr, bool do_an, 
 // stepLitePrimary and computeIntegratedDepthDoseLite, proxy 0.
 template <typename T>
 cudaError_t enq_lite_step(bfpn_ctx* c) {
-    const int trap = (c->p.flags & BFPN_FLAG_TRAPEZOIDAL_YZ) ? 1 : 0;
-    const int n = lite_energy_grid(c->per_e);
-    cudaError_t e = prof(c, BFPN_KERNEL_ENERGY, [&] {
-        return launch_lite_energy<T>(as<T>(c->st[0][0]), c->lite_coef, c->d.dt, c->Ng, c->per_e, c->dose_coef, c->NA,
-                                     c->Ny, c->Nz, trap, c->partials, c->stream);
-    });
+    EnergyArgs<T> a{};
+    a.F = as<T>(c->st[0][0]);
+    a.coef = c->lite_coef;
+    a.Ng = c->Ng;
+    a.lanes = c->per_e;
+    a.partials = c->partials;
+    a.dose_coef = c->dose_coef;
+    a.NA = c->NA;
+    a.Ny = c->Ny;
+    a.Nz = c->Nz;
+    a.trapezoidal = (c->p.flags & BFPN_FLAG_TRAPEZOIDAL_YZ) ? 1 : 0;
+    const int n = energy_grid(c->elem, c->per_e, c->NA, true, true);  // consecutive lanes
+    cudaError_t e = prof(c, BFPN_KERNEL_ENERGY, [&] { return launch_lite_energy<T>(a, c->stream); });
     if (e != cudaSuccess) return e;
     const double w = c->d.du * c->d.dv * c->d.dy * c->d.dz;
     return prof(c, BFPN_KERNEL_IDD, [&] {

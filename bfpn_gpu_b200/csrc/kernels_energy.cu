@@ -547,6 +547,81 @@ __global__ void __launch_bounds__(kEnergyMaxLanes / LPT) energy_fused_kernel(Ene
     if (dose) block_partials(acc, accp, a.partials + 2 * bid);
 }
 
+// ---------------------------------------------------------------------------
+// Lite-memory primary step (litePrimaryEnergyStepKernel, bfpm_solver.cu:593-620):
+// psi^1 only, first-order upwind in energy with catastrophic attenuation,
+// groups swept from Ng-1 down, in place:
+//   F_g <- max((max(F_g,0)/dt + S_hi/dg * F_{g+1}) / max(denom, eps), 0)
+// as max(k max(F_g, 0) + h F_{g+1}, 0) with the constants (k, h) of a group
+// formed once on the host: the two FP64 divisions of a group were the serial
+// chain (21 x 21 x 400 lanes, 500 groups, float: 0.88 ms a step against 0.11 ms
+// of HBM traffic).  The IDD of the new state (Eq. 24 with psi^2 = 0,
+// integratedDepthDoseLiteKernel, bfpm_solver.cu:523-591) is accumulated on the
+// way as per-block partials; the psi^2 column is 0.
+// ---------------------------------------------------------------------------
+template <typename T, int LPT, bool CS>
+__global__ void __launch_bounds__(kEnergyMaxLanes / LPT) lite_energy_kernel(EnergyArgs<T> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int U = RingShape<LPT>::U, DB = RingShape<LPT>::D / U;
+    using R = Ring<T, LPT, 1>;
+    const int Ng = a.Ng;
+    const LaneSpan span = lane_span<T, LPT>(a, blockIdx.x, false);
+    const long long L = a.lanes, lane0 = span.lane0;
+    const bool ok = span.ok;
+    R ring;
+    ring.L = L;
+    ring.Ng = Ng;
+    ring.ok = ok;
+    ring.src[0] = a.F + lane0;
+    ring.base = reinterpret_cast<typename R::V*>(smem_raw + energy_table_bytes(Ng, 1, true, CS));
+    ring.start();
+    double2* tab = reinterpret_cast<double2*>(smem_raw);  // [Ng] (k, h), then [Ng] dose weights
+    const double2* gk = reinterpret_cast<const double2*>(a.coef);
+    const double2* gd = reinterpret_cast<const double2*>(a.dose_coef);
+    if (CS) {
+        for (int e = threadIdx.x; e < Ng; e += blockDim.x) {
+            tab[e] = __ldg(gk + e);
+            tab[Ng + e] = __ldg(gd + e);
+        }
+        __syncthreads();
+    }
+    double w[LPT], next[LPT], acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < LPT; ++j) {
+        w[j] = lane_weight(a, lane0 + j);
+        next[j] = 0.0;
+    }
+    auto trip_of = [&](auto FULLc, int t) {
+        constexpr bool full = decltype(FULLc)::value;
+        ring.template wait<false>(t);
+        const int k0 = (t % DB) * U, e0 = Ng - 1 - t * U;
+        T F[U][LPT];
+#pragma unroll
+        for (int u = 0; u < U; ++u) unpack(*ring.slot(k0 + u, 0), F[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int ek = e0 - u;
+            if (!full && ek < 0) break;
+            const double2 c = CS ? tab[ek] : __ldg(gk + ek);
+            const double dose = CS ? tab[Ng + ek].x : __ldg(gd + ek).x;
+            T Fs[LPT];
+#pragma unroll
+            for (int j = 0; j < LPT; ++j) {
+                Fs[j] = static_cast<T>(fmax(fma(c.y, next[j], c.x * fmax(static_cast<double>(F[u][j]), 0.0)), 0.0));
+                next[j] = static_cast<double>(Fs[j]);
+                if (ok) acc = fma(w[j] * dose, next[j], acc);
+            }
+            if (ok) store_lanes(a.F + static_cast<size_t>(ek) * L + lane0, Fs);
+        }
+    };
+    const int full_trips = Ng / U;
+#pragma unroll 1
+    for (int t = 0; t < full_trips; ++t) trip_of(std::true_type(), t);
+    if (Ng % U) trip_of(std::false_type(), full_trips);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    block_partials(acc, 0.0, a.partials + 2 * static_cast<long long>(blockIdx.x));
+}
+
 // ---- launch shapes ----------------------------------------------------------
 // Lanes per thread: vectors once they leave four warps for each SM; a vector
 // never straddles two positions.
@@ -637,6 +712,19 @@ cudaError_t launch_fused(const EnergyFusedArgs& A, cudaStream_t s) {
         [&](size_t b) { return go(energy_fused_kernel<MODE, false, LPT>, b); });
 }
 
+template <typename T, int LPT>
+cudaError_t launch_lite(const EnergyArgs<T>& a, cudaStream_t s) {
+    const PassShape sh = pass_shape(sizeof(T), a.lanes, a.NA, LPT, false);
+    const size_t ring = ring_bytes<LPT, T>(sh.threads, 1), tab = energy_table_bytes(a.Ng, 1, true, true);
+    const bool cs = tab + ring <= kEnergySmemLimit;
+    auto kern = cs ? lite_energy_kernel<T, LPT, true> : lite_energy_kernel<T, LPT, false>;
+    const size_t smem = cs ? tab + ring : ring;
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+    if (e != cudaSuccess) return e;
+    kern<<<sh.grid, sh.threads, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 int energy_grid(size_t elem, long long lanes, int NA, bool src, bool dose, int lanes_per_thread) {
@@ -672,6 +760,14 @@ cudaError_t launch_energy(const EnergyArgs<T>& a, cudaStream_t s) {
 }
 template cudaError_t launch_energy<float>(const EnergyArgs<float>&, cudaStream_t);
 template cudaError_t launch_energy<double>(const EnergyArgs<double>&, cudaStream_t);
+
+template <typename T>
+cudaError_t launch_lite_energy(const EnergyArgs<T>& a, cudaStream_t s) {
+    constexpr int V = sizeof(T) == 4 ? 4 : 2;
+    return vector_lanes(sizeof(T), a.lanes, a.NA) == V ? launch_lite<T, V>(a, s) : launch_lite<T, 1>(a, s);
+}
+template cudaError_t launch_lite_energy<float>(const EnergyArgs<float>&, cudaStream_t);
+template cudaError_t launch_lite_energy<double>(const EnergyArgs<double>&, cudaStream_t);
 
 cudaError_t launch_energy_slots(const EnergyArgs<float>* args, const int* begin, int nslots, int blocks, int mode,
                                 bool vec, bool src, bool dose, int max_ng, long long lanes, int NA, cudaStream_t s) {

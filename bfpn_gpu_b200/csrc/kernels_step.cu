@@ -1,5 +1,4 @@
-// Depth-step kernels: the lite-memory energy step, MUSCL predictor-corrector
-// transport, separable DST-I angular diffusion, IDD
+// Depth-step kernels: MUSCL predictor-corrector transport, separable DST-I angular diffusion, IDD
 // finalisation, beam initialisation and conversions.
 //
 // State layout (HBM): index = (ek * nyz + pos) * NA + ang, ang fastest, the
@@ -49,74 +48,6 @@ cudaError_t allow_dynamic_smem(const void* func, size_t need) {
 
 template <typename T>
 cudaError_t launch_angle_generic(const AngleArgs<T>& a, cudaStream_t s);
-
-// ---------------------------------------------------------------------------
-// Lite-memory primary step (litePrimaryEnergyStepKernel, bfpm_solver.cu:593-620):
-// psi^1 only, first-order upwind in energy with catastrophic attenuation,
-// groups swept from Ng-1 down, in place:
-//   F_g <- max((max(F_g,0)/dt + S_hi/dg * F_{g+1}) / max(denom, eps), 0)
-// with the per-group S_hi/dg and max(denom, eps) precomputed in double in the
-// reference's operation order.  The IDD of the new state (Eq. 24 with psi^2 = 0,
-// integratedDepthDoseLiteKernel, bfpm_solver.cu:523-591) is accumulated on the
-// way as per-block partials; the psi^2 column is 0.
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(128) lite_energy_kernel(T* __restrict__ F, const double* __restrict__ lc, double dt,
-                                                          int Ng, long long lanes, const double* __restrict__ dc,
-                                                          int NA, int Ny, int Nz, int trap, double* partials) {
-    constexpr int D = 8;  // groups prefetched ahead of use
-    const long long lane = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const bool ok = lane < lanes;
-    T ring[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-        const int e = Ng - 1 - k;
-        ring[k] = (ok && e >= 0) ? F[e * lanes + lane] : T(0);
-    }
-    double w = 1.0;
-    if (trap && ok) {
-        const int pos = static_cast<int>(lane / NA), iy = pos % (Ny + 1), iz = pos / (Ny + 1);
-        if (iy == 0 || iy == Ny) w *= 0.5;
-        if (iz == 0 || iz == Nz) w *= 0.5;
-    }
-    double next = 0.0, acc = 0.0;
-    for (int base = Ng - 1; base >= 0; base -= D)
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-        const int ek = base - k;
-        if (ek < 0) break;
-        const double Fg = fmax(static_cast<double>(ring[k]), 0.0);
-        const int ep = ek - D;
-        if (ep >= 0 && ok) ring[k] = F[ep * lanes + lane];
-        const double v = fmax((Fg / dt + __ldg(lc + 2 * ek) * next) / __ldg(lc + 2 * ek + 1), 0.0);
-        const T vs = static_cast<T>(v);
-        if (ok) {
-            F[ek * lanes + lane] = vs;
-            acc += w * __ldg(dc + 2 * ek) * static_cast<double>(vs);
-        }
-        next = static_cast<double>(vs);
-    }
-    __shared__ double red[4];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    const int wi = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) red[wi] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0.0;
-        for (int i = 0; i < static_cast<int>(blockDim.x >> 5); ++i) a += red[i];
-        partials[2 * blockIdx.x] = a;
-        partials[2 * blockIdx.x + 1] = 0.0;
-    }
-}
-
-int lite_energy_grid(long long lanes) { return static_cast<int>((lanes + 127) / 128); }
-
-template <typename T>
-cudaError_t launch_lite_energy(T* F, const double* lc, double dt, int Ng, long long lanes, const double* dc, int NA,
-                               int Ny, int Nz, int trap, double* partials, cudaStream_t s) {
-    lite_energy_kernel<T><<<lite_energy_grid(lanes), 128, 0, s>>>(F, lc, dt, Ng, lanes, dc, NA, Ny, Nz, trap, partials);
-    return cudaGetLastError();
-}
 
 // ---------------------------------------------------------------------------
 // Lateral transport, Eq. (18) (spatial_transport.cu:23-161, 202-262).
@@ -2408,8 +2339,6 @@ cudaError_t launch_convert(const Tin* in, Tout* out, long long n, cudaStream_t s
 }
 
 #define BFPN_INSTANTIATE(T)                                                                                       \
-    template cudaError_t launch_lite_energy<T>(T*, const double*, double, int, long long, const double*, int, int,  \
-                                               int, int, double*, cudaStream_t);                                  \
     template cudaError_t launch_transport<T>(const TransportArgs<T>&, int, cudaStream_t);                         \
     template cudaError_t launch_transport_plane<T>(const TransportArgs<T>&, int, cudaStream_t);                   \
     template cudaError_t launch_transport_tiles<T>(const TransportArgs<T>&, int, cudaStream_t);                   \

@@ -502,9 +502,9 @@ std::vector<double> lite_coefficients(const BeamTables& t, double dt) {
     for (int ek = 0; ek < t.Ng; ++ek) {
         const double sig = std::max(t.sigma[ek], 0.0);
         const double S_lo = std::max(t.S_s[ek], 0.0), S_hi = std::max(t.S_s[ek + 1], 0.0);
-        const double denom = 1.0 / dt + S_lo / dg + sig;
-        c[2 * ek] = S_hi / dg;
-        c[2 * ek + 1] = std::max(denom, kEpsilon);
+        const double denom = std::max(1.0 / dt + S_lo / dg + sig, kEpsilon);
+        c[2 * ek] = 1.0 / dt / denom;
+        c[2 * ek + 1] = S_hi / dg / denom;
     }
     return c;
 }
