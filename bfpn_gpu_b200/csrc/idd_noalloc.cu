@@ -23,6 +23,8 @@
 #include "common.cuh"
 #include "tables.hpp"
 
+#include <algorithm>
+#include <cstdint>
 #include <string>
 
 using namespace bfpn;
@@ -49,7 +51,13 @@ static __device__ __align__(256) unsigned char g_idd_scratch[kScratchBytes];
 
 namespace {
 
-template <typename T>
+// The pass reads the arrays once and is HBM-bound, so it needs bytes in flight:
+// a block takes 1024 lanes of a share of the groups (blockIdx.y) in 16-byte
+// pieces, with as many shares as fill eight blocks per SM.  (One lane and one
+// group at a time per thread, on 173 blocks, read the 21 x 21 x 400-lane, 500
+// group float state at 1.2 TB/s; this form reads it at the rate in the design
+// notes' table.)  VEC: the arrays and rows are 16-byte aligned.
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(kThreads) idd_noalloc_kernel(const T* __restrict__ F0, const T* __restrict__ f0,
                                                                const T* __restrict__ F1, const T* __restrict__ f1,
                                                                const double* __restrict__ dc, int Ng, long long lanes,
@@ -58,25 +66,55 @@ __global__ void __launch_bounds__(kThreads) idd_noalloc_kernel(const T* __restri
                                                                double* out) {
     unsigned int* ticket = reinterpret_cast<unsigned int*>(scratch);
     double* part = reinterpret_cast<double*>(scratch + kHeaderBytes);
+    constexpr int W = VEC ? static_cast<int>(16 / sizeof(T)) : 1, PIECES = kLanesPerThread / W;
+    using V = typename Vec16<T>::type;
+    const int share = (Ng + gridDim.y - 1) / gridDim.y, e0 = blockIdx.y * share, e1 = min(Ng, e0 + share);
+    const unsigned int n_blocks = gridDim.x * gridDim.y, block = blockIdx.y * gridDim.x + blockIdx.x;
     double acc = 0.0, accp = 0.0;
-    for (int k = 0; k < kLanesPerThread; ++k) {
-        const long long lane = static_cast<long long>(blockIdx.x) * kLanesPerBlock + k * kThreads + threadIdx.x;
-        if (lane >= lanes) break;
-        double w = 1.0;
-        if (trap) {
-            const int pos = static_cast<int>(lane / NA), iy = pos % (Ny + 1), iz = pos / (Ny + 1);
-            if (iy == 0 || iy == Ny) w *= 0.5;
-            if (iz == 0 || iz == Nz) w *= 0.5;
-        }
-        double d = 0.0;
-        for (int ek = 0; ek < Ng; ++ek) {
+#pragma unroll
+    for (int k = 0; k < PIECES; ++k) {
+        const long long lane = static_cast<long long>(blockIdx.x) * kLanesPerBlock + (k * kThreads + threadIdx.x) * W;
+        if (lane >= lanes) break;  // VEC: lanes is a multiple of W
+        double d[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) d[j] = 0.0;
+        auto add = [&](const T* A, long long i, double c, bool proxy) {
+            T x[W];
+            if constexpr (VEC) {
+                const V v = __ldcs(reinterpret_cast<const V*>(A + i));
+#pragma unroll
+                for (int j = 0; j < W; ++j) x[j] = reinterpret_cast<const T*>(&v)[j];
+            } else {
+                x[0] = A[i];
+            }
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+                const double y = static_cast<double>(x[j]);
+                d[j] = fma(c, y, d[j]);
+                if (proxy) accp += y;
+            }
+        };
+#pragma unroll 2
+        for (int ek = e0; ek < e1; ++ek) {
             const long long i = ek * lanes + lane;
-            const double x = static_cast<double>(F0[i]), y = static_cast<double>(f0[i]);
-            d += dc[2 * ek] * x + dc[2 * ek + 1] * y;
-            accp += y;
-            if (F1) d += dc[2 * ek] * static_cast<double>(F1[i]) + dc[2 * ek + 1] * static_cast<double>(f1[i]);
+            const double c1 = __ldg(dc + 2 * ek), c2 = __ldg(dc + 2 * ek + 1);
+            add(F0, i, c1, false);
+            add(f0, i, c2, true);
+            if (F1) {
+                add(F1, i, c1, false);
+                add(f1, i, c2, false);
+            }
         }
-        acc += w * d;
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            double w = 1.0;
+            if (trap) {
+                const int pos = static_cast<int>((lane + j) / NA), iy = pos % (Ny + 1), iz = pos / (Ny + 1);
+                if (iy == 0 || iy == Ny) w *= 0.5;
+                if (iz == 0 || iz == Nz) w *= 0.5;
+            }
+            acc += w * d[j];
+        }
     }
     __shared__ double red[2][kThreads / 32];
     __shared__ bool last;
@@ -90,17 +128,17 @@ __global__ void __launch_bounds__(kThreads) idd_noalloc_kernel(const T* __restri
     if (threadIdx.x == 0) {
         double a = 0.0, b = 0.0;
         for (int i = 0; i < kThreads / 32; ++i) { a += red[0][i]; b += red[1][i]; }
-        part[2 * blockIdx.x] = a;
-        part[2 * blockIdx.x + 1] = b;
+        part[2 * block] = a;
+        part[2 * block + 1] = b;
         __threadfence();  // the pair is visible device-wide before the ticket is taken
-        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        last = atomicAdd(ticket, 1u) == n_blocks - 1;
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
     const volatile double* vp = part;
     double a = 0.0, b = 0.0;
-    for (int i = threadIdx.x; i < static_cast<int>(gridDim.x); i += kThreads) { a += vp[2 * i]; b += vp[2 * i + 1]; }
+    for (int i = threadIdx.x; i < static_cast<int>(n_blocks); i += kThreads) { a += vp[2 * i]; b += vp[2 * i + 1]; }
     for (int o = 16; o > 0; o >>= 1) {
         a += __shfl_down_sync(0xffffffffu, a, o);
         b += __shfl_down_sync(0xffffffffu, b, o);
@@ -183,21 +221,30 @@ extern "C" bfpn_status bfpn_idd_noalloc(const bfpn_grid* grid, int32_t precision
 
     const Deltas d = compute_deltas(g);
     const double idd_scale = d.du * d.dv * d.dy * d.dz;
-    const int blocks = static_cast<int>((lanes + kLanesPerBlock - 1) / kLanesPerBlock);
+    const int lane_blocks = static_cast<int>((lanes + kLanesPerBlock - 1) / kLanesPerBlock);
+    // eight blocks per SM; at least 8 groups each, and no more pairs than the scratch holds
+    const int shares = std::max(1, std::min({148 * 8 / lane_blocks, g.Ng / 8, kMaxBlocks / lane_blocks}));
+    const dim3 blocks(static_cast<unsigned>(lane_blocks), static_cast<unsigned>(shares));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     e = cudaMemsetAsync(scratch, 0, sizeof(unsigned int), s);  // the ticket counter starts at zero
     if (e != cudaSuccess) return noalloc_fail(BFPN_CUDA_ERROR, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
     const int trap = trapezoidal_yz ? 1 : 0;
-    if (precision == BFPN_PREC_FP64)
-        idd_noalloc_kernel<double><<<blocks, kThreads, 0, s>>>(
-            static_cast<const double*>(F0), static_cast<const double*>(f0), static_cast<const double*>(F1),
-            static_cast<const double*>(f1), dose_coef, g.Ng, lanes, static_cast<int>(NA), g.Ny, g.Nz, trap, idd_scale,
-            d.dg, scratch, out);
-    else
-        idd_noalloc_kernel<float><<<blocks, kThreads, 0, s>>>(
-            static_cast<const float*>(F0), static_cast<const float*>(f0), static_cast<const float*>(F1),
-            static_cast<const float*>(f1), dose_coef, g.Ng, lanes, static_cast<int>(NA), g.Ny, g.Nz, trap, idd_scale,
-            d.dg, scratch, out);
+    // the caller's arrays may start anywhere a T may
+    auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    const bool rows16 = aligned(F0) && aligned(f0) && aligned(F1) && aligned(f1);
+    auto go = [&](auto zero, auto kern) {
+        using T = decltype(zero);
+        kern<<<blocks, kThreads, 0, s>>>(static_cast<const T*>(F0), static_cast<const T*>(f0), static_cast<const T*>(F1),
+                                         static_cast<const T*>(f1), dose_coef, g.Ng, lanes, static_cast<int>(NA), g.Ny,
+                                         g.Nz, trap, idd_scale, d.dg, scratch, out);
+    };
+    if (precision == BFPN_PREC_FP64) {
+        if (rows16 && lanes % 2 == 0) go(0.0, idd_noalloc_kernel<double, true>);
+        else go(0.0, idd_noalloc_kernel<double, false>);
+    } else {
+        if (rows16 && lanes % 4 == 0) go(0.f, idd_noalloc_kernel<float, true>);
+        else go(0.f, idd_noalloc_kernel<float, false>);
+    }
     e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(BFPN_CUDA_ERROR, std::string("idd_noalloc_kernel: ") + cudaGetErrorString(e));
     return BFPN_OK;

@@ -125,3 +125,32 @@ def test_lite_step_shapes(ny, nz, nmu, nom, ng, precision):
     # (two groups lose the beam within the steps: float values end below 2^-126, where a rounding is 2^-150)
     floor = 0.0 if precision == capi.PREC_FP64 else 6 * 2.0 ** -149
     assert np.abs(a - b).max() <= tol * np.abs(b).max() + floor
+
+
+# 16-byte pieces and not (a caller's array may start at any value; odd lane
+# counts), fewer groups than one share, with and without the secondary
+@pytest.mark.parametrize("dtype,precision", [(torch.float64, capi.PREC_FP64), (torch.float32, capi.PREC_MIXED)])
+@pytest.mark.parametrize("ny,nz,nmu,nom,ng,shift", [(2, 2, 3, 3, 3, 0), (6, 5, 4, 6, 41, 0), (6, 5, 4, 6, 41, 1),
+                                                    (20, 21, 12, 12, 19, 0), (4, 4, 5, 5, 100, 2)])
+def test_caller_owned_dose_shapes(ny, nz, nmu, nom, ng, shift, dtype, precision):
+    cfg = small_cfg(ny=ny, nz=nz, nmu=nmu, nom=nom, ng=ng, trapezoidal_yz=True)
+    g = cfg.grid()
+    n = ng * (ny + 1) * (nz + 1) * nmu * nom
+    rng = torch.Generator(device="cuda").manual_seed(5)
+    own = [torch.rand(n + shift, device="cuda", dtype=dtype, generator=rng)[shift:] for _ in range(4)]
+    w = torch.rand(2 * ng, device="cuda", dtype=torch.float64, generator=rng)
+    wy, wz = np.ones(ny + 1), np.ones(nz + 1)
+    wy[[0, -1]], wz[[0, -1]] = 0.5, 0.5
+    pos = torch.from_numpy((wz[:, None] * wy[None, :]).ravel()).cuda()[None, :, None]
+    F0, f0, F1, f1 = [a.double().view(ng, -1, nmu * nom) for a in own]
+    k = w.view(ng, 2, 1, 1)
+    vol = g.Ly / ny * g.Lz / nz * g.Lu / (nom + 1) * g.Lv / (nmu + 1)
+    for second in (True, False):
+        out = torch.zeros(2, device="cuda", dtype=torch.float64)
+        ptr = [a.data_ptr() for a in own]
+        capi.idd_noalloc(g, precision, True, ptr[0], ptr[1], ptr[2] if second else None, ptr[3] if second else None,
+                         w.data_ptr(), out.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+        psi1, psi2 = (F0 + F1, f0 + f1) if second else (F0, f0)
+        want = [float(((k[:, 0] * psi1 + k[:, 1] * psi2) * pos).sum()) * vol, float(f0.sum()) * g.Lg / ng]
+        # sums of at most 2e7 positive terms in double: 1e-11 covers any order
+        assert np.allclose(out.cpu().numpy(), want, rtol=1e-11, atol=0.0)
