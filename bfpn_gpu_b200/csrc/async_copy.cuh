@@ -87,6 +87,11 @@ __device__ __forceinline__ void cp_async_ca(void* dst, const void* src) {
     else
         asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
 }
+// An 8-byte copy; an invalid piece is filled with zeros (nothing is read).
+__device__ __forceinline__ void cp_async8(void* dst, const void* src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 8 : 0)
+                 : "memory");
+}
 // A 16-byte copy under a predicate (no branch, nothing written when off).
 __device__ __forceinline__ void cp_async16_if(void* dst, const void* src, bool on) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(

@@ -467,7 +467,10 @@ cudaError_t enq_source_on(bfpn_ctx* c, const void* P1, const void* P2, void* S, 
                                              c->e_et, c->e_emax, as<float>(S), c->dev_err, per_e, c->Ng, c->stream);
         });
     }
-    e = prof(c, BFPN_KERNEL_SOURCE_ANGULAR, [&] { return launch_source_angular<T>(a, c->stream); });
+    e = prof(c, BFPN_KERNEL_SOURCE_ANGULAR, [&] {
+        if constexpr (sizeof(T) == 8) return launch_source_angular_f64(a, c->kmask, c->stream);
+        else return launch_source_angular<T>(a, c->stream);
+    });
     if (e != cudaSuccess) return e;
     if (pread && (e = cudaEventRecord(pread, c->stream)) != cudaSuccess) return e;
     return prof(c, BFPN_KERNEL_SOURCE_ENERGY, [&] { return launch_source_energy<T>(a, c->tile_e, c->stream); });
@@ -1561,6 +1564,7 @@ bfpn_status bfpn_load_tables(bfpn_ctx* c, const double* mu, int32_t mu_rows, con
     dfree(c, c->bblob);
     dfree(c, c->eblob);
     { void* w = c->ulist; dfree(c, w); c->ulist = nullptr; }
+    { void* w = c->kmask; dfree(c, w); c->kmask = nullptr; }
     { void* w = c->ubegin; dfree(c, w); c->ubegin = nullptr; }
     { void* w = c->ework; dfree(c, w); c->ework = nullptr; }
     { void* w = c->ework_begin; dfree(c, w); c->ework_begin = nullptr; }
@@ -1568,6 +1572,12 @@ bfpn_status bfpn_load_tables(bfpn_ctx* c, const double* mu, int32_t mu_rows, con
     // beam's tables may have had a kernel there
     if (c->A1) CUDA_TRY(c, cudaMemsetAsync(c->A1, 0, c->a_bytes, c->stream));
     c->ooc_ready = false;  // the chunk buffers depend on the source groups
+    if (c->prec == BFPN_PREC_FP64 && c->ker_v && !groups.empty()) {
+        void* m = nullptr;
+        if ((s = dalloc(c, &m, source_mask_bytes(c->n_groups, c->NA))) != BFPN_OK) return s;
+        c->kmask = static_cast<uint32_t*>(m);
+        CUDA_TRY(c, launch_source_mask(as<const double>(c->ker_v), c->groups, c->n_groups, c->NA, c->kmask, c->stream));
+    }
     if (c->prec == BFPN_PREC_MIXED && (c->A1 || (c->ooc && c->ker_v)) && !groups.empty()) {
         // tensor-core source: output tiles of <= 256 columns, multiples of 16
         c->umma_ntiles = (c->NA + 255) / 256;

@@ -197,6 +197,11 @@ template <typename T> cudaError_t launch_angle(const AngleArgs<T>& a, cudaStream
 // Any angular grid up to 32 x 32 (kernels_dst.cu).
 template <typename T> cudaError_t launch_angle_rect(const AngleArgs<T>& a, cudaStream_t s);
 template <typename T> cudaError_t launch_source_angular(const SourceArgs<T>& a, cudaStream_t s);
+// FP64 angular stage over the non-zero 8 x 32 blocks of the kernel, marked in
+// mask (source_mask_bytes, launch_source_mask once per table load).
+cudaError_t launch_source_angular_f64(const SourceArgs<double>& a, const uint32_t* mask, cudaStream_t s);
+cudaError_t launch_source_mask(const double* ker_v, const int* groups, int n_groups, int NA, uint32_t* mask, cudaStream_t s);
+size_t source_mask_bytes(int n_groups, int NA);
 template <typename T> cudaError_t launch_source_energy(const SourceArgs<T>& a, int tile_e, cudaStream_t s);
 template <typename T> cudaError_t launch_init_beam(T* F, const double* yza, const double* e, long long per_e,
                                                    int Ng, cudaStream_t s);

@@ -73,6 +73,7 @@ struct bfpn_ctx {
     int* ubegin = nullptr;          // [n_groups * umma_ntiles + 1] offsets into ulist
     int* ework = nullptr;           // energy work items {chunk, column, columns, e group}
     int* ework_begin = nullptr;     // [e tiles + 1]
+    uint32_t* kmask = nullptr;      // FP64: non-zero blocks of the angular kernel
     int e_et = 0, e_emax = 0;
     bool use_umma = true;
     int umma_nt = 0, umma_bk = 16, umma_ntiles = 0;

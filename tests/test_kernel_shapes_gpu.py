@@ -109,6 +109,21 @@ def test_rectangular_angle_shapes(nom, nmu, precision):
     assert_states(ctx, ora, OP_TOL if precision == capi.PREC_FP64 else 2e-5)
 
 
+# odd and even angle counts, partial 32-output tiles and 8-row chunks, positions
+# around one 64-position tile; the last grid's kernel has zero blocks
+@pytest.mark.parametrize("ny,nz,nmu,nom,ng,tables", [(3, 4, 3, 3, 40, "synthetic500"), (7, 7, 5, 7, 40, "synthetic500"),
+                                                     (8, 6, 8, 8, 40, "synthetic500"), (2, 2, 20, 20, 500, "water")])
+def test_fp64_source_shapes(ny, nz, nmu, nom, ng, tables):
+    cfg = small_cfg(ny=ny, nz=nz, nmu=nmu, nom=nom, ng=ng, lg=0.518 * ng if ng == 500 else 59.0,
+                    beam_energy=230.0 if ng == 500 else 40.0)
+    ctx, ora = build(cfg, tables=tables)
+    set_both(ctx, ora, seeded_states(ctx, 44))
+    ctx.secondary_source()
+    s = ora.source()
+    assert np.abs(s).max() > 0
+    assert rel_err(ctx.source(), s) < OP_TOL
+
+
 @pytest.mark.parametrize("precision", PRECISIONS)
 @pytest.mark.parametrize("ny,nz,nmu,nom,ng", [(2, 3, 3, 3, 2), (6, 5, 4, 5, 43), (17, 17, 16, 16, 9)])
 def test_lite_step_shapes(ny, nz, nmu, nom, ng, precision):
