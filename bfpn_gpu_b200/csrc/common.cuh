@@ -214,6 +214,9 @@ cudaError_t launch_finalize_idd(const double* partials, int n, const double* par
                                 double idd_scale, double proxy_scale, double* hist_idd,
                                 double* hist_proxy, int* counter, int capacity, int advance,
                                 cudaStream_t s);
+// count history values and the error word into mapped host memory.
+cudaError_t launch_export_history(const double* idd, const double* proxy, int count, const int* err, double* idd_out,
+                                  double* proxy_out, int* err_out, cudaStream_t s);
 // Stand-alone IDD partials of one species (F, f) when it was not fused into
 // an energy pass.  partials: [grid][2].
 template <typename T>

@@ -2215,6 +2215,22 @@ __global__ void __launch_bounds__(1024) finalize_idd_slots_kernel(const IddFinal
     }
 }
 
+__global__ void __launch_bounds__(256) export_history_kernel(const double* __restrict__ idd, const double* __restrict__ proxy,
+                                                             int count, const int* err, double* idd_out, double* proxy_out,
+                                                             int* err_out) {
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        idd_out[i] = idd[i];
+        proxy_out[i] = proxy[i];
+    }
+    if (threadIdx.x == 0) *err_out = *err;
+}
+
+cudaError_t launch_export_history(const double* idd, const double* proxy, int count, const int* err, double* idd_out,
+                                  double* proxy_out, int* err_out, cudaStream_t s) {
+    export_history_kernel<<<1, 256, 0, s>>>(idd, proxy, count, err, idd_out, proxy_out, err_out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_finalize_idd_slots(const IddFinalArgs* args, int nslots, cudaStream_t s) {
     if (nslots <= 0) return cudaSuccess;
     finalize_idd_slots_kernel<<<nslots, 1024, 0, s>>>(args);
