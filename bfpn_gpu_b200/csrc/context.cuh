@@ -64,6 +64,7 @@ struct bfpn_ctx {
     double* hist_proxy = nullptr;
     int hist_cap = 0;
     int* counter = nullptr;
+    void* stage[2] = {};            // pinned buffers of large state transfers (in host_allocs)
     void* step_export = nullptr;    // pinned, mapped: results of one step call (in host_allocs)
     int* zero_counter = nullptr;    // scratch counter for one-off IDD reductions
     int* dev_err = nullptr;         // device error word (bounded waits that ran out)
