@@ -133,11 +133,13 @@ __device__ __forceinline__ double flip(double x, double s) {
     return __longlong_as_double(__double_as_longlong(x) ^
                                 (__double_as_longlong(s) & static_cast<long long>(0x8000000000000000ull)));
 }
-__device__ __forceinline__ double march_limit(double back, double back2, double fwd, double fwd2) {
-    const double b = flip(back, fwd), b2 = flip(back2, fwd), af = fabs(fwd), af2 = fabs(fwd2);
-    const double lo = b2 < af ? b2 : af, hi = b < af2 ? b : af2;
-    const double m = lo > hi ? lo : hi;
-    return flip(m > 0.0 ? m : 0.0, fwd);
+// Same signs: min(max(|back|, |fwd|), 2 min(|back|, |fwd|)).
+__device__ __forceinline__ double march_limit(double back, double, double fwd, double) {
+    const double ab = fabs(back), af = fabs(fwd);
+    const bool less = ab < af;
+    const double lo = less ? ab : af, hi = less ? af : ab, lo2 = lo + lo;
+    const double m = hi < lo2 ? hi : lo2;
+    return (__double2hiint(back) ^ __double2hiint(fwd)) >= 0 ? flip(m, fwd) : 0.0;
 }
 __device__ __forceinline__ double march_keep(double cut) { return fabs(cut) >= kEpsilon ? 1.0 : 0.0; }
 
