@@ -558,7 +558,10 @@ cudaError_t enq_source_on(bfpn_ctx* c, const void* P1, const void* P2, void* S, 
     });
     if (e != cudaSuccess) return e;
     if (pread && (e = cudaEventRecord(pread, c->stream)) != cudaSuccess) return e;
-    return prof(c, BFPN_KERNEL_SOURCE_ENERGY, [&] { return launch_source_energy<T>(a, c->tile_e, c->stream); });
+    return prof(c, BFPN_KERNEL_SOURCE_ENERGY, [&] {
+        if constexpr (sizeof(T) == 8) return launch_source_energy_f64(a, c->band8, c->stream);
+        else return launch_source_energy(a, c->tile_e, c->stream);
+    });
 }
 
 template <typename T>
@@ -1584,6 +1587,7 @@ bfpn_status bfpn_create(const bfpn_grid* grid, const bfpn_phys* phys, int precis
     ALLOC(c->gmap, static_cast<size_t>(c->Ng) * sizeof(int));
     ALLOC(c->tile_lo, static_cast<size_t>(c->Ng) * sizeof(int));
     ALLOC(c->tile_hi, static_cast<size_t>(c->Ng) * sizeof(int));
+    ALLOC(c->band8, (static_cast<size_t>(c->Ng) + 7) / 8 * sizeof(int2));
     ALLOC(c->beam_yza, static_cast<size_t>(c->per_e) * sizeof(double));
     ALLOC(c->beam_e, static_cast<size_t>(c->Ng) * sizeof(double));
     // [primary, even steps | secondary | primary, odd steps] x n_part x 2
@@ -1781,6 +1785,13 @@ bfpn_status bfpn_load_tables(bfpn_ctx* c, const double* mu, int32_t mu_rows, con
             hi[tI] = h;
         }
     }
+    std::vector<int2> band8((c->Ng + 7) / 8, make_int2(c->Ng, 0));
+    for (int e = 0; e < c->Ng; ++e)
+        if (T.band_end[e] > T.band_begin[e]) {
+            int2& b = band8[e / 8];
+            b = make_int2(std::min(b.x, T.band_begin[e]), std::max(b.y, T.band_end[e]));
+        }
+    if ((s = upload_f64(c, c->band8, band8.data(), band8.size() * sizeof(int2))) != BFPN_OK) return s;
     if ((s = upload_f64(c, c->tile_lo, lo.data(), lo.size() * sizeof(int))) != BFPN_OK) return s;
     if ((s = upload_f64(c, c->tile_hi, hi.data(), hi.size() * sizeof(int))) != BFPN_OK) return s;
     if ((s = upload_f64(c, c->beam_yza, T.beam_yza.data(), T.beam_yza.size() * sizeof(double))) != BFPN_OK) return s;

@@ -202,7 +202,10 @@ template <typename T> cudaError_t launch_source_angular(const SourceArgs<T>& a, 
 cudaError_t launch_source_angular_f64(const SourceArgs<double>& a, const uint32_t* mask, cudaStream_t s);
 cudaError_t launch_source_mask(const double* ker_v, const int* groups, int n_groups, int NA, uint32_t* mask, cudaStream_t s);
 size_t source_mask_bytes(int n_groups, int NA);
-template <typename T> cudaError_t launch_source_energy(const SourceArgs<T>& a, int tile_e, cudaStream_t s);
+cudaError_t launch_source_energy(const SourceArgs<float>& a, int tile_e, cudaStream_t s);
+// FP64 energy stage; band8: the union band [first, last) of the source groups of
+// each 8 output groups.
+cudaError_t launch_source_energy_f64(const SourceArgs<double>& a, const int2* band8, cudaStream_t s);
 template <typename T> cudaError_t launch_init_beam(T* F, const double* yza, const double* e, long long per_e,
                                                    int Ng, cudaStream_t s);
 

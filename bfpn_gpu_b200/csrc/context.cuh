@@ -75,6 +75,7 @@ struct bfpn_ctx {
     int* ubegin = nullptr;          // [n_groups * umma_ntiles + 1] offsets into ulist
     int* ework = nullptr;           // energy work items {chunk, column, columns, e group}
     int* ework_begin = nullptr;     // [e tiles + 1]
+    int2* band8 = nullptr;          // FP64: union band of each 8 output groups
     uint32_t* kmask = nullptr;      // FP64: non-zero blocks of the angular kernel
     int e_et = 0, e_emax = 0;
     bool use_umma = true;

@@ -243,6 +243,109 @@ __global__ void __launch_bounds__(128) source_angular_f64_kernel(SourceArgs<doub
     }
 }
 
+// ---------------------------------------------------------------------------
+// FP64 energy stage on the double tensor instruction.  A block computes 32 output
+// groups x 64 lanes, a warp 8 of the groups: per k = 4 step 16 m8n8k4 products
+// for both operands.  The source groups of the 32 outputs' union band stream
+// through three cp.async stages, 8 at a time; a warp multiplies only the chunks
+// its own 8 outputs' band meets (band8).  Coefficients and values are read once
+// per block from L2, blocks of one lane range next to each other.  Against 16
+// output groups per SIMT thread, whose every multiply-add loaded its coefficient
+// from shared memory: 441 positions x 400 angles x 500 groups 1.75 -> 1.06 ms,
+// 121 x 121 x 500 0.168 -> 0.128 ms, 289 x 64 x 200 0.073 -> 0.050 ms.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(128) source_energy_f64_kernel(SourceArgs<double> a, const int2* __restrict__ band8) {
+    constexpr int BE = 32, BN = 64, BK = 8, EP = 12, VP = 68, NST = 3;
+    __shared__ __align__(16) double Es[NST][2][BE][EP];
+    __shared__ __align__(16) double Vs[NST][2][BK][VP];
+    const int Ng = a.Ng, n_et = (Ng + BE - 1) / BE, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int e0 = static_cast<int>(blockIdx.x % n_et) * BE;
+    const long long per_e = static_cast<long long>(a.nyz) * a.NA, l0 = static_cast<long long>(blockIdx.x / n_et) * BN;
+    int lo = Ng, hi = 0;
+    int2 own = make_int2(0, 0);
+    for (int w = 0; w < BE / 8; ++w) {
+        if (e0 + 8 * w >= Ng) break;
+        const int2 b = __ldg(band8 + e0 / 8 + w);
+        if (w == warp) own = b;
+        if (b.x < b.y) {
+            lo = min(lo, b.x);
+            hi = max(hi, b.y);
+        }
+    }
+    const int n = hi > lo ? (hi - lo + BK - 1) / BK : 0;
+    const bool vec = per_e % 2 == 0;  // rows on 16-byte boundaries
+    auto fill = [&](int i) {          // source groups lo + 8 i .. of the band into stage i % NST
+        if (i < n) {
+            const int s0 = lo + i * BK, st = i % NST;
+            for (int v = tid; v < 2 * BE * BK; v += 128) {
+                const int k = v % BK, e = (v / BK) % BE, op = v / (BK * BE), s = s0 + k;
+                const bool in = s < hi && e0 + e < Ng;
+                const double* E = op ? a.e2 : a.e1;
+                cp_async8(&Es[st][op][e][k], in ? E + static_cast<size_t>(e0 + e) * Ng + s : E, in);
+            }
+            const int per = vec ? BN / 2 : BN, step = vec ? 2 : 1;
+            for (int v = tid; v < 2 * BK * per; v += 128) {
+                const int c = (v % per) * step, k = (v / per) % BK, op = v / (per * BK), s = s0 + k;
+                const bool in = s < hi && l0 + c < per_e;
+                const double* A = op ? a.A2 : a.A1;
+                const double* src = in ? A + s * per_e + l0 + c : A;
+                if (vec) cp_async16(&Vs[st][op][k][c], src, in);
+                else cp_async8(&Vs[st][op][k][c], src, in);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double acc[2][BN / 8][2];
+#pragma unroll
+    for (int op = 0; op < 2; ++op)
+#pragma unroll
+        for (int nt = 0; nt < BN / 8; ++nt) acc[op][nt][0] = acc[op][nt][1] = 0.0;
+    for (int i = 0; i < NST - 1; ++i) fill(i);
+    const int r = lane >> 2, q = lane & 3;
+    for (int i = 0; i < n; ++i) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(NST - 2) : "memory");
+        __syncthreads();  // chunk i has landed for every thread; chunk i - 1's stage is free
+        fill(i + NST - 1);
+        const int st = i % NST, s0 = lo + i * BK;
+        if (s0 >= own.y || s0 + BK <= own.x) continue;  // zero coefficients for this warp's outputs
+#pragma unroll
+        for (int k4 = 0; k4 < BK; k4 += 4) {
+#pragma unroll
+            for (int op = 0; op < 2; ++op) {
+                const double ev = Es[st][op][warp * 8 + r][k4 + q];
+                double bv[BN / 8];
+#pragma unroll
+                for (int nt = 0; nt < BN / 8; ++nt) bv[nt] = Vs[st][op][k4 + q][nt * 8 + r];
+#pragma unroll
+                for (int nt = 0; nt < BN / 8; ++nt) dmma(acc[op][nt], ev, bv[nt]);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    const int e = e0 + warp * 8 + r;
+    if (e >= Ng) return;
+    const double dg = a.dg, third = 1.0 / 3.0;
+#pragma unroll
+    for (int nt = 0; nt < BN / 8; ++nt) {
+        const long long l = l0 + nt * 8 + 2 * q;
+        const double v0 = dg * (acc[0][nt][0] + acc[1][nt][0] * third), v1 = dg * (acc[0][nt][1] + acc[1][nt][1] * third);
+        double* o = a.S + e * per_e + l;
+        if (vec && l < per_e) {
+            *reinterpret_cast<double2*>(o) = make_double2(v0, v1);
+        } else {
+            if (l < per_e) o[0] = v0;
+            if (l + 1 < per_e) o[1] = v1;
+        }
+    }
+}
+
+cudaError_t launch_source_energy_f64(const SourceArgs<double>& a, const int2* band8, cudaStream_t s) {
+    const long long per_e = static_cast<long long>(a.nyz) * a.NA, blocks = (per_e + 63) / 64 * ((a.Ng + 31) / 32);
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    source_energy_f64_kernel<<<static_cast<unsigned>(blocks), 128, 0, s>>>(a, band8);
+    return cudaGetLastError();
+}
+
 int source_mask_words(int NA) { return ((NA + kMaskRows - 1) / kMaskRows + 31) / 32; }
 size_t source_mask_bytes(int n_groups, int NA) {
     return static_cast<size_t>(n_groups) * ((NA + kMaskCols - 1) / kMaskCols) * source_mask_words(NA) * sizeof(uint32_t);
@@ -337,102 +440,21 @@ __global__ void __launch_bounds__(128) source_energy_f2_kernel(SourceArgs<float>
         }
 }
 
-// Energy stage: TE output groups per block and LN lanes per thread.  The
-// source groups of the union band of the TE outputs are streamed once; the
-// band coefficients of a chunk of SC source groups are staged in shared
-// memory as [s][t] rows (one vector broadcast load feeds 4 (float) or 2
-// (double) accumulators), and zeros outside an output's own band add
-// nothing.  Accumulation in the state precision; blockIdx.x walks the output
-// tiles so blocks sharing a lane range run together and share A rows in L2.
-template <typename T, int TE, int LN>
-__global__ void __launch_bounds__(128) source_energy_kernel(SourceArgs<T> a) {
-    constexpr int SC = 32;
-    __shared__ __align__(16) T E1[SC][TE];
-    __shared__ __align__(16) T E2[SC][TE];
-    const int tile = blockIdx.x;
-    const long long per_e = static_cast<long long>(a.nyz) * a.NA;
-    const long long l0 = static_cast<long long>(blockIdx.y) * blockDim.x * LN + threadIdx.x;
-    const int Ng = a.Ng, e0 = tile * TE;
-    const int lo = a.tile_lo[tile], hi = a.tile_hi[tile];
-    T q1[TE][LN], q2[TE][LN];
-#pragma unroll
-    for (int t = 0; t < TE; ++t)
-#pragma unroll
-        for (int j = 0; j < LN; ++j) { q1[t][j] = T(0); q2[t][j] = T(0); }
-    long long lj[LN];
-    bool ok[LN];
-#pragma unroll
-    for (int j = 0; j < LN; ++j) {
-        lj[j] = l0 + static_cast<long long>(j) * blockDim.x;
-        ok[j] = lj[j] < per_e;
-    }
-    for (int s0 = lo; s0 < hi; s0 += SC) {
-        const int n = min(SC, hi - s0);
-        __syncthreads();
-        for (int k = threadIdx.x; k < SC * TE; k += blockDim.x) {
-            const int ss = k / TE, t = k - ss * TE, e = e0 + t;
-            const bool in = ss < n && e < Ng;
-            E1[ss][t] = in ? static_cast<T>(a.e1[static_cast<size_t>(e) * Ng + s0 + ss]) : T(0);
-            E2[ss][t] = in ? static_cast<T>(a.e2[static_cast<size_t>(e) * Ng + s0 + ss]) : T(0);
-        }
-        __syncthreads();
-#pragma unroll 2
-        for (int ss = 0; ss < n; ++ss) {
-            T x1[LN], x2[LN];
-            const long long row = static_cast<long long>(s0 + ss) * per_e;
-#pragma unroll
-            for (int j = 0; j < LN; ++j) {
-                x1[j] = ok[j] ? a.A1[row + lj[j]] : T(0);
-                x2[j] = ok[j] ? a.A2[row + lj[j]] : T(0);
-            }
-#pragma unroll
-            for (int t = 0; t < TE; ++t) {
-                const T c1 = E1[ss][t], c2 = E2[ss][t];
-#pragma unroll
-                for (int j = 0; j < LN; ++j) {
-                    q1[t][j] += c1 * x1[j];
-                    q2[t][j] += c2 * x2[j];
-                }
-            }
-        }
-    }
-    const T dg = static_cast<T>(a.dg), third = T(1) / T(3);
-#pragma unroll
-    for (int t = 0; t < TE; ++t) {
-        const int e = e0 + t;
-        if (e >= Ng) continue;
-#pragma unroll
-        for (int j = 0; j < LN; ++j)
-            if (ok[j]) a.S[e * per_e + lj[j]] = dg * (q1[t][j] + q2[t][j] * third);
-    }
-}
-
-template <typename T>
-cudaError_t launch_source_energy(const SourceArgs<T>& a, int tile_e, cudaStream_t s) {
-    constexpr int LN = sizeof(T) == 4 ? 2 : 1;
+cudaError_t launch_source_energy(const SourceArgs<float>& a, int tile_e, cudaStream_t s) {
+    constexpr int LN = 2;
     const long long per_e = static_cast<long long>(a.nyz) * a.NA;
     const int tiles = (a.Ng + tile_e - 1) / tile_e;
     const long long ly = (per_e + 128 * LN - 1) / (128 * LN);
     if (ly > 65535) return cudaErrorInvalidConfiguration;
     dim3 grid(tiles, static_cast<unsigned>(ly));
-    if constexpr (sizeof(T) == 4) {
-        switch (tile_e) {
-            case 8: source_energy_f2_kernel<8, LN><<<grid, 128, 0, s>>>(a); break;
-            case 16: source_energy_f2_kernel<16, LN><<<grid, 128, 0, s>>>(a); break;
-            default: return cudaErrorInvalidValue;
-        }
-    } else {
-        switch (tile_e) {
-            case 8: source_energy_kernel<T, 8, LN><<<grid, 128, 0, s>>>(a); break;
-            case 16: source_energy_kernel<T, 16, LN><<<grid, 128, 0, s>>>(a); break;
-            default: return cudaErrorInvalidValue;
-        }
+    switch (tile_e) {
+        case 8: source_energy_f2_kernel<8, LN><<<grid, 128, 0, s>>>(a); break;
+        case 16: source_energy_f2_kernel<16, LN><<<grid, 128, 0, s>>>(a); break;
+        default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 
 template cudaError_t launch_source_angular<float>(const SourceArgs<float>&, cudaStream_t);
-template cudaError_t launch_source_energy<double>(const SourceArgs<double>&, int, cudaStream_t);
-template cudaError_t launch_source_energy<float>(const SourceArgs<float>&, int, cudaStream_t);
 
 }  // namespace bfpn
