@@ -156,6 +156,21 @@ __global__ void __launch_bounds__(256) pack_source_operand_kernel(UmmaPackArgs a
     *reinterpret_cast<uint4*>(base + a_part + off) = lo;
 }
 
+// 16 accumulator columns of the warp's 32 rows; v is valid after
+// tcgen05.wait::ld, and settle16 ties it to that wait.
+__device__ __forceinline__ void tmem_load16(uint32_t addr, uint32_t* v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(addr));
+}
+__device__ __forceinline__ void settle16(uint32_t* v) {
+    asm volatile(""
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]),
+                   "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]));
+}
+
 struct UmmaPipeArgs {
     const uint8_t* ablob;
     const uint8_t* bblob;    // [n_groups][n_ntiles][nk][hi|lo][N_T x BK bf16, core layout]
@@ -191,6 +206,19 @@ __global__ void __launch_bounds__(128, 1) source_angular_umma_pipe_kernel(UmmaPi
         return a.ulist ? __ldg(a.ulist + u0 + it) : make_int4(it, 0, NT, 0);
     };
 
+    const uint8_t* __restrict__ ablob = a.ablob + (static_cast<size_t>(gz) * a.n_mt + mt) * a.nk * (2 * a_part);
+    const uint8_t* __restrict__ bblob =
+        a.bblob + (static_cast<size_t>(gz) * a.n_ntiles + nt) * a.nk * static_cast<size_t>(2 * b_part);
+    int issued[kPipe] = {};  // thread 0's
+    auto issue = [&](int it) {
+        const int st = it % kPipe;
+        const int kc = entry(it).x;
+        uint8_t* sA = smem + st * stage_bytes;
+        mbar_expect_tx(&bar_full[st], 2 * a_part + 2 * b_part);
+        bulk_copy_g2s(sA, ablob + static_cast<size_t>(kc) * 2 * a_part, 2 * a_part, &bar_full[st]);
+        bulk_copy_g2s(sA + 2 * a_part, bblob + static_cast<size_t>(kc) * 2 * b_part, 2 * b_part, &bar_full[st]);
+        ++issued[st];
+    };
     if (tid == 0) {
         for (int s = 0; s < kPipe; ++s) {
             mbar_init(&bar_full[s], 1);
@@ -198,6 +226,9 @@ __global__ void __launch_bounds__(128, 1) source_angular_umma_pipe_kernel(UmmaPi
         }
         mbar_init_fence();
         fail_flag = 0;
+        // the first chunks fly while tensor memory is allocated (which may wait
+        // for another CTA's) and zeroed
+        for (int it = 0; it < min(kPipe, nk); ++it) issue(it);
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
@@ -225,24 +256,11 @@ __global__ void __launch_bounds__(128, 1) source_angular_umma_pipe_kernel(UmmaPi
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-    const uint8_t* __restrict__ ablob = a.ablob + (static_cast<size_t>(gz) * a.n_mt + mt) * a.nk * (2 * a_part);
-    const uint8_t* __restrict__ bblob =
-        a.bblob + (static_cast<size_t>(gz) * a.n_ntiles + nt) * a.nk * static_cast<size_t>(2 * b_part);
     const uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kRows >> 4) << 24);
 
     if (tid == 0) {
-        int issued[kPipe] = {}, landed[kPipe] = {}, committed[kPipe] = {}, drained[kPipe] = {};
-        auto issue = [&](int it) {
-            const int st = it % kPipe;
-            const int kc = entry(it).x;
-            uint8_t* sA = smem + st * stage_bytes;
-            mbar_expect_tx(&bar_full[st], 2 * a_part + 2 * b_part);
-            bulk_copy_g2s(sA, ablob + static_cast<size_t>(kc) * 2 * a_part, 2 * a_part, &bar_full[st]);
-            bulk_copy_g2s(sA + 2 * a_part, bblob + static_cast<size_t>(kc) * 2 * b_part, 2 * b_part, &bar_full[st]);
-            ++issued[st];
-        };
+        int landed[kPipe] = {}, committed[kPipe] = {}, drained[kPipe] = {};
         bool bad = false;
-        for (int it = 0; it < min(kPipe, nk); ++it) issue(it);
         for (int it = 0; it < nk && !bad; ++it) {
             const int st = it % kPipe;
             if (!mbar_wait(&bar_full[st], (it / kPipe) & 1)) {
@@ -300,32 +318,41 @@ __global__ void __launch_bounds__(128, 1) source_angular_umma_pipe_kernel(UmmaPi
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (!fail_flag) {
-        // Epilogue through shared memory (the pipeline buffers are free now):
-        // 16-column slices of the accumulator go to a [128][17]-float tile;
-        // then each thread takes 8 consecutive outputs of one row, splits
-        // them into bf16 hi / lo and writes both into the energy operand
-        // layout.  Two threads share a row, so with 8-aligned lanes one warp
-        // store covers whole 32-byte pieces.
-        float* tile = reinterpret_cast<float*>(smem);
-        constexpr int TS = 17;  // padded row stride
+        // Epilogue: a warp owns the accumulator's rows 32 warp .. 32 warp + 31
+        // and works alone (through block-wide steps the four warps waited for
+        // each other twice per 16 columns, most of the kernel's time).  Slices
+        // of 32 columns go to the warp's own [32][33]-float tile (the pipeline
+        // buffers are free now); then each lane takes 8 consecutive outputs of
+        // a row, splits them into bf16 hi / lo and writes both into the energy
+        // operand layout, four lanes per row, so a warp store covers whole
+        // 32-byte sectors, 64 bytes of a row.
+        constexpr int TS = 33;  // padded row stride
+        const int lane = tid & 31;
+        float* tile = reinterpret_cast<float*>(smem) + warp * 32 * TS;
         const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-        for (int c0 = 0; c0 < NT; c0 += 16) {
-            uint32_t v[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                : "r"(tmem + lane_base + c0));
+        const int plane = warp >= 2 ? 2 : 0;
+        for (int c0 = 0; c0 < NT; c0 += 32) {
+            const int pieces = NT - c0 >= 32 ? 4 : 2;  // NT is a multiple of 16
+            uint32_t v[32];
+            tmem_load16(tmem + lane_base + c0, v);
+            if (pieces == 4) tmem_load16(tmem + lane_base + c0 + 16, v + 16);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            settle16(v);
+            if (pieces == 4) settle16(v + 16);
 #pragma unroll
-            for (int q = 0; q < 16; ++q) tile[tid * TS + q] = __uint_as_float(v[q]);
-            __syncthreads();
-            for (int task = tid; task < 2 * kRows; task += 128) {
-                const int r = task >> 1, h = task & 1;
-                const int pos = m0 + (r & (kPos - 1));
+            for (int q = 0; q < 16; ++q) tile[lane * TS + q] = __uint_as_float(v[q]);
+            if (pieces == 4) {
+#pragma unroll
+                for (int q = 16; q < 32; ++q) tile[lane * TS + q] = __uint_as_float(v[q]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (i >= pieces) break;
+                const int task = i * 32 + lane, r = pieces == 4 ? task >> 2 : task >> 1, h = task & (pieces - 1);
+                const int pos = m0 + ((warp * 32 + r) & (kPos - 1));
                 const int n = n0 + c0 + 8 * h;
                 if (pos >= a.nyz || n >= a.NA) continue;
-                const int plane = r >= kPos ? 2 : 0;
                 const long long l = static_cast<long long>(pos) * a.NA + n;
                 const float* x = tile + r * TS + 8 * h;
                 if ((l & 7) == 0 && n + 8 <= a.NA) {
@@ -339,18 +366,20 @@ __global__ void __launch_bounds__(128, 1) source_angular_umma_pipe_kernel(UmmaPi
                                                 pack_bf16(y[6], y[7]));
                     const uint4 lo = make_uint4(pack_bf16(z[0], z[1]), pack_bf16(z[2], z[3]), pack_bf16(z[4], z[5]),
                                                 pack_bf16(z[6], z[7]));
-                    *reinterpret_cast<uint4*>(a.q + q_offset(plane, g, l, a.nsg)) = hi;
-                    *reinterpret_cast<uint4*>(a.q + q_offset(plane + 1, g, l, a.nsg)) = lo;
+                    uint8_t* o = a.q + q_offset(plane, g, l, a.nsg);
+                    *reinterpret_cast<uint4*>(o) = hi;
+                    *reinterpret_cast<uint4*>(o + 2048) = lo;  // the next plane
                 } else {
                     for (int k = 0; k < 8 && n + k < a.NA; ++k) {
                         const __nv_bfloat16 hb = __float2bfloat16_rn(x[k]);
                         const __nv_bfloat16 lb = __float2bfloat16_rn(x[k] - __bfloat162float(hb));
-                        *reinterpret_cast<__nv_bfloat16*>(a.q + q_offset(plane, g, l + k, a.nsg)) = hb;
-                        *reinterpret_cast<__nv_bfloat16*>(a.q + q_offset(plane + 1, g, l + k, a.nsg)) = lb;
+                        uint8_t* o = a.q + q_offset(plane, g, l + k, a.nsg);
+                        *reinterpret_cast<__nv_bfloat16*>(o) = hb;
+                        *reinterpret_cast<__nv_bfloat16*>(o + 2048) = lb;
                     }
                 }
             }
-            __syncthreads();
+            __syncwarp();
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -447,6 +476,19 @@ __global__ void __launch_bounds__(128, 1) source_energy_umma_kernel(EnergyUmmaAr
     const uint32_t raw = smem_u32(smem);
     uint8_t* stages = smem + (((raw + 1023u) & ~1023u) - raw);
 
+    int issued[kMaxStagesE] = {};  // thread 0's
+    const uint8_t* __restrict__ qtile = a.q + static_cast<size_t>(lt) * a.nsg * 8192;
+    auto issue = [&](int it) {
+        const int st = it % nst;
+        const int4 w = a.work[w0 + it];
+        uint8_t* sQ = stages + st * a.stage_bytes;
+        const uint32_t ebytes = static_cast<uint32_t>(w.z) * 128u;  // columns x 4 planes x 16 groups x 2 B
+        mbar_expect_tx(&bar_full[st], kQStage + ebytes);
+        bulk_copy_g2s(sQ, qtile + static_cast<size_t>(2 * w.x) * 8192, kQStage, &bar_full[st]);
+        bulk_copy_g2s(sQ + kQStage, a.eblob + (static_cast<size_t>(w.x) * a.n_eg + w.w) * 1024, ebytes,
+                      &bar_full[st]);
+        ++issued[st];
+    };
     if (tid == 0) {
         for (int st = 0; st < nst; ++st) {
             mbar_init(&bar_full[st], 1);
@@ -454,6 +496,8 @@ __global__ void __launch_bounds__(128, 1) source_energy_umma_kernel(EnergyUmmaAr
         }
         mbar_init_fence();
         fail_flag = 0;
+        // the first chunks fly while tensor memory is allocated and zeroed
+        for (int it = 0; it < min(nst, nw); ++it) issue(it);
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
@@ -481,24 +525,10 @@ __global__ void __launch_bounds__(128, 1) source_energy_umma_kernel(EnergyUmmaAr
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     if (tid == 0 && nw > 0) {
-        int issued[kMaxStagesE] = {}, landed[kMaxStagesE] = {}, committed[kMaxStagesE] = {},
-            drained[kMaxStagesE] = {};
-        const uint8_t* __restrict__ qtile = a.q + static_cast<size_t>(lt) * a.nsg * 8192;
-        auto issue = [&](int it) {
-            const int st = it % nst;
-            const int4 w = a.work[w0 + it];
-            uint8_t* sQ = stages + st * a.stage_bytes;
-            const uint32_t ebytes = static_cast<uint32_t>(w.z) * 128u;  // columns x 4 planes x 16 groups x 2 B
-            mbar_expect_tx(&bar_full[st], kQStage + ebytes);
-            bulk_copy_g2s(sQ, qtile + static_cast<size_t>(2 * w.x) * 8192, kQStage, &bar_full[st]);
-            bulk_copy_g2s(sQ + kQStage, a.eblob + (static_cast<size_t>(w.x) * a.n_eg + w.w) * 1024, ebytes,
-                          &bar_full[st]);
-            ++issued[st];
-        };
+        int landed[kMaxStagesE] = {}, committed[kMaxStagesE] = {}, drained[kMaxStagesE] = {};
         constexpr uint32_t idesc_base = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) |
                                         (static_cast<uint32_t>(128 >> 4) << 24);  // f32 += bf16 x bf16, A MN-major
         bool bad = false;
-        for (int it = 0; it < min(nst, nw); ++it) issue(it);
         for (int it = 0; it < nw && !bad; ++it) {
             const int st = it % nst;
             if (!mbar_wait(&bar_full[st], (it / nst) & 1)) {
@@ -554,17 +584,16 @@ __global__ void __launch_bounds__(128, 1) source_energy_umma_kernel(EnergyUmmaAr
         const int ncol = min(kEnergyCols, a.Ng - E0);
         const long long l = lt * 128 + tid;  // accumulator row tid = lane tid of the tile
         float* __restrict__ S = a.S + static_cast<size_t>(E0) * a.per_e + l;
-        for (int c0 = 0; c0 < ncol; c0 += 16) {
-            uint32_t v[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                : "r"(tmem + lane_base + c0));
+        for (int c0 = 0; c0 < ncol; c0 += 32) {
+            uint32_t v[32];
+            tmem_load16(tmem + lane_base + c0, v);
+            tmem_load16(tmem + lane_base + c0 + 16, v + 16);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            settle16(v);
+            settle16(v + 16);
             if (l < a.per_e) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
+                for (int j = 0; j < 32; ++j)
                     if (c0 + j < ncol) S[static_cast<size_t>(c0 + j) * a.per_e] = __uint_as_float(v[j]);
             }
         }
