@@ -256,10 +256,17 @@ cudaError_t launch_source_angular_pipe(const float* P1, const float* P2, uint8_t
                                        const int* groups, int n_groups, uint8_t* q, int Ng, int* err, int nyz,
                                        int NA, int NT, int BK, int n_ntiles, const int4* ulist, const int* ubegin,
                                        cudaStream_t s, cudaEvent_t packed = nullptr, bool pack = true);
-// Host: the entries of ulist / ubegin from the float angular kernel kv
-// ([Ng][NA in][NA out]) of the source groups.
-void build_umma_ranges(const float* kv, const int* groups, int n_groups, int NA, int NT, int BK, int n_ntiles,
-                       std::vector<int4>& list, std::vector<int>& begin);
+// Host: the entries of ulist / ubegin from the non-zero column ranges of
+// launch_angular_ranges ([n_groups][n_ntiles][nk]).
+void build_umma_ranges(const int2* ranges, int n_groups, int NT, int nk, int n_ntiles, std::vector<int4>& list,
+                       std::vector<int>& begin);
+// The angular kernel table ([Ng][NA][NA]) from the directions ([NA][2]) and the
+// scattering rows ([Ng][3]), all on the device (kernels_tables.cu).
+template <typename T>
+cudaError_t launch_angular_kernel(const double* omega, const double* mu, int NA, int Ng, T* ker_v, cudaStream_t s);
+// Non-zero column range [x, y) of each BK-row chunk of each NT-column tile.
+cudaError_t launch_angular_ranges(const float* ker_v, const int* groups, int n_groups, int NA, int NT, int BK, int n_ntiles,
+                                  int2* ranges, cudaStream_t s);
 size_t umma_pack_bytes(int n_groups, int nyz, int NA, int BK);
 size_t umma_q_bytes(long long per_e, int Ng);
 // Tensor-core energy stage: S[e][l] from q with the coefficient tiles and

@@ -738,31 +738,17 @@ __global__ void build_umma_blob_kernel(const float* __restrict__ ker_v, const in
     *reinterpret_cast<uint4*>(base + part + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
 }
 
-void build_umma_ranges(const float* kv, const int* groups, int n_groups, int NA, int NT, int BK, int n_ntiles,
-                       std::vector<int4>& list, std::vector<int>& begin) {
-    const int nk = (NA + BK - 1) / BK;
+void build_umma_ranges(const int2* ranges, int n_groups, int NT, int nk, int n_ntiles, std::vector<int4>& list,
+                       std::vector<int>& begin) {
     list.clear();
     begin.assign(static_cast<size_t>(n_groups) * n_ntiles + 1, 0);
-    for (int gz = 0; gz < n_groups; ++gz) {
-        const float* K = kv + static_cast<size_t>(groups[gz]) * NA * NA;  // [in][out]
-        for (int nt = 0; nt < n_ntiles; ++nt) {
-            begin[static_cast<size_t>(gz) * n_ntiles + nt] = static_cast<int>(list.size());
-            const int n0 = nt * NT, n1 = std::min(NA, n0 + NT);
-            for (int kc = 0; kc < nk; ++kc) {
-                int lo = NT, hi = 0;
-                for (int in = kc * BK; in < std::min(NA, (kc + 1) * BK); ++in) {
-                    const float* row = K + static_cast<size_t>(in) * NA;
-                    for (int o = n0; o < n1; ++o)
-                        if (row[o] != 0.0f) {
-                            lo = std::min(lo, o - n0);
-                            hi = std::max(hi, o - n0 + 1);
-                        }
-                }
-                if (hi <= lo) continue;
-                lo = lo / 16 * 16;
-                hi = std::min(NT, (hi + 15) / 16 * 16);
-                list.push_back(make_int4(kc, lo, hi - lo, 0));
-            }
+    for (size_t tile = 0; tile + 1 < begin.size(); ++tile) {
+        begin[tile] = static_cast<int>(list.size());
+        for (int kc = 0; kc < nk; ++kc) {
+            const int2 r = ranges[tile * nk + kc];
+            if (r.y <= r.x) continue;
+            const int lo = r.x / 16 * 16, hi = std::min(NT, (r.y + 15) / 16 * 16);
+            list.push_back(make_int4(kc, lo, hi - lo, 0));
         }
     }
     begin.back() = static_cast<int>(list.size());
