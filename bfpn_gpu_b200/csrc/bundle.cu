@@ -38,6 +38,7 @@ using namespace bfpn;
 namespace {
 
 constexpr int kMaxSideStreams = 4;
+constexpr int kTuneSteps = 6;        // depth steps of one tuning run
 constexpr int kBundleMaxPlane = 65;  // Ny + 1 and Nz + 1 of a bundle's beams
 
 struct Tuning {
@@ -349,9 +350,12 @@ bfpn_status ensure_plan(bfpn_bundle* b, const std::vector<int>& prim, const std:
     return BFPN_OK;
 }
 
-// Autotuning: two eager steps per variant set, A and B alternating (A B A B),
-// each kernel class keeps its faster variant.  The steps are real steps of
-// the bundle.  Returns the steps taken.
+// Autotuning: three eager steps per variant set, A and B alternating (A B A B
+// A B), each kernel class keeps its faster variant by the last pair: the steps
+// before load the code of its kernels (the secondary's from the second step on),
+// which takes up to 30 ms and would decide the choice.  Beams too short for
+// that run set A untuned.  The steps are real steps of the bundle.  Returns the
+// steps taken.
 bfpn_status autotune(bfpn_bundle* b, const std::vector<int>& prim, int max_steps, int* taken) {
     *taken = 0;
     Tuning A = b->tune, B = b->tune;
@@ -361,8 +365,8 @@ bfpn_status autotune(bfpn_bundle* b, const std::vector<int>& prim, int max_steps
     B.dst_stages = 3;
     A.ring = true;
     B.ring = false;
-    double tA[TK_N] = {}, tB[TK_N] = {};
-    const int rounds = std::min(4, max_steps);
+    double warm[TK_N] = {}, tA[TK_N] = {}, tB[TK_N] = {};
+    const int rounds = std::min(kTuneSteps, max_steps);
     for (int r = 0; r < rounds; ++r) {
         b->tune = (r % 2 == 0) ? A : B;
         // a slot's first step has no secondary half
@@ -371,14 +375,14 @@ bfpn_status autotune(bfpn_bundle* b, const std::vector<int>& prim, int max_steps
             if (b->slots[s].ctx->steps_done > 0) sec_now.push_back(s);
         bfpn_status st = ensure_plan(b, prim, sec_now, false);
         if (st != BFPN_OK) return st;
-        cudaError_t e = enq_bundle_step(b, (r % 2 == 0) ? tA : tB);
+        cudaError_t e = enq_bundle_step(b, r < 4 ? warm : (r % 2 == 0) ? tA : tB);
         if (e != cudaSuccess) return bfail(b, BFPN_CUDA_ERROR, std::string("bundle tuning step: ") + cudaGetErrorString(e));
         for (int s : prim) b->slots[s].ctx->steps_done += 1;
         ++*taken;
         b->plan_sig.clear();
     }
     Tuning best = A;
-    if (rounds >= 2) {
+    if (rounds == kTuneSteps) {
         const bool fixed_tr = b->cl || b->march;  // one transport form: nothing to choose
         best.tr_ac = (fixed_tr || tA[TK_TRANSPORT] <= tB[TK_TRANSPORT]) ? A.tr_ac : B.tr_ac;
         best.dst_stages = tA[TK_ANGLE] <= tB[TK_ANGLE] ? A.dst_stages : B.dst_stages;
@@ -386,7 +390,7 @@ bfpn_status autotune(bfpn_bundle* b, const std::vector<int>& prim, int max_steps
         best.tuned = true;
         char buf[320];
         std::snprintf(buf, sizeof buf,
-                      "%s: transport %s (%.3f ms vs %.3f ms per step-pair), DST %d stages (%.3f vs %.3f), "
+                      "%s: transport %s (%.3f ms vs %.3f ms per step), DST %d stages (%.3f vs %.3f), "
                       "energy %s (%.3f vs %.3f)",
                       b->key.c_str(),
                       b->march ? "marching" : b->cl ? "cluster" : (best.tr_ac == 16 ? "16 angles/block" : "8 angles/block"),
@@ -570,7 +574,7 @@ bfpn_status bfpn_bundle_step(bfpn_bundle* b, int32_t nsteps) {
             min_rest = std::min(min_rest, s.nsteps - s.ctx->steps_done);
         }
         if (prim.empty()) break;
-        if (b->autotune && !b->tune.tuned) {
+        if (b->autotune && !b->tune.tuned && min_rest >= kTuneSteps) {
             int taken = 0;
             bfpn_status st = autotune(b, prim, min_rest, &taken);
             if (st != BFPN_OK) return st;

@@ -278,9 +278,11 @@ void choose_transport(bfpn_ctx* c) {
 // The unrolled whole-plane kernel, where one is compiled for this plane
 // size; it works in place whatever the line-walk kernel's shape.
 void choose_plane_transport(bfpn_ctx* c) {
-    // 16 float / 4 double angles per block: 64 / 32 contiguous bytes per position
-    // (16 float angles measured 7% faster than 8 on a 21x21 plane)
-    c->tr_plane_ac = c->elem == 4 ? 16 : 4;
+    // float: 16 angles per block (64 contiguous bytes per position) while three
+    // such blocks share an SM, else 8.  Measured per launch, 16 / 8 angles:
+    // 21 x 21 x 400 angles 2.66 / 2.82 ps per cell, 25 x 25 x 256 3.33 / 3.16,
+    // 33 x 33 x 256 4.29 / 3.51.  Double: 4 angles
+    c->tr_plane_ac = c->elem == 8 ? 4 : 3 * transport_plane_smem(c->Ny + 1, 16, c->elem) <= 216 * 1024 ? 16 : 8;
     c->tr_plane_ok = transport_plane_supported(c->Ny, c->Nz) &&
                      transport_plane_smem(c->Ny + 1, c->tr_plane_ac, c->elem) <= 200 * 1024;
     c->tr_plane = c->tr_plane_ok;
@@ -1646,9 +1648,7 @@ bfpn_status bfpn_load_tables(bfpn_ctx* c, const double* mu, int32_t mu_rows, con
     if (s != BFPN_OK) return s;
     std::string err;
     BeamTables t;
-    // a float-state context keeps only the float angular kernel on the host
-    const bool f32_kernel = c->prec == BFPN_PREC_MIXED;
-    if (!build_tables(c->g, c->p, mu, mu_rows, sigma_c, sigma_rows, t, err, f32_kernel))
+    if (!build_tables(c->g, c->p, mu, mu_rows, sigma_c, sigma_rows, t, err, false))
         return fail(c, BFPN_INVALID_ARG, err);
     c->tables = std::move(t);
     c->raw_sigma.assign(sigma_c, sigma_c + std::min<int>(sigma_rows, c->Ng));
@@ -1666,13 +1666,13 @@ bfpn_status bfpn_load_tables(bfpn_ctx* c, const double* mu, int32_t mu_rows, con
     if ((s = upload_state_table(c, c->sine_u, T.sine_u)) != BFPN_OK) return s;
     if ((s = upload_state_table(c, c->sine_v, T.sine_v)) != BFPN_OK) return s;
     if (c->ker_v) {
-        if (f32_kernel) {
-            CUDA_TRY(c, cudaMemcpyAsync(c->ker_v, T.ker_v_f.data(), T.ker_v_f.size() * sizeof(float),
-                                        cudaMemcpyHostToDevice, c->stream));
-            CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-        } else if ((s = upload_state_table(c, c->ker_v, T.ker_v)) != BFPN_OK) {
-            return s;
-        }
+        // its inputs in double, in buffers whose own contents come later
+        // (beam_yza: nyz NA values, nyz >= 4; ecoef_op: rebuilt for each dt)
+        if ((s = upload_f64(c, c->beam_yza, T.omega.data(), T.omega.size() * sizeof(double))) != BFPN_OK) return s;
+        if ((s = upload_f64(c, c->ecoef_op, T.mu.data(), T.mu.size() * sizeof(double))) != BFPN_OK) return s;
+        CUDA_TRY(c, c->prec == BFPN_PREC_FP64
+                        ? launch_angular_kernel(c->beam_yza, c->ecoef_op, c->NA, c->Ng, as<double>(c->ker_v), c->stream)
+                        : launch_angular_kernel(c->beam_yza, c->ecoef_op, c->NA, c->Ng, as<float>(c->ker_v), c->stream));
     }
     if ((s = upload_f64(c, c->e1, T.ker_e1.data(), T.ker_e1.size() * sizeof(double))) != BFPN_OK) return s;
     if ((s = upload_f64(c, c->e2, T.ker_e2.data(), T.ker_e2.size() * sizeof(double))) != BFPN_OK) return s;
@@ -1739,11 +1739,19 @@ bfpn_status bfpn_load_tables(bfpn_ctx* c, const double* mu, int32_t mu_rows, con
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
         // the kernel blocks' non-zero k chunks and column ranges (the kernel is
         // sparse: entries below the threshold were dropped)
-        if (!T.ker_v_f.empty()) {
+        {
+            const int nk = (c->NA + c->umma_bk - 1) / c->umma_bk;
+            std::vector<int2> ranges(static_cast<size_t>(c->n_groups) * c->umma_ntiles * nk);
+            void* dr = nullptr;
+            if ((s = dalloc(c, &dr, ranges.size() * sizeof(int2))) != BFPN_OK) return s;
+            CUDA_TRY(c, launch_angular_ranges(as<const float>(c->ker_v), c->groups, c->n_groups, c->NA, c->umma_nt, c->umma_bk,
+                                              c->umma_ntiles, static_cast<int2*>(dr), c->stream));
+            CUDA_TRY(c, cudaMemcpyAsync(ranges.data(), dr, ranges.size() * sizeof(int2), cudaMemcpyDeviceToHost, c->stream));
+            CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+            dfree(c, dr);
             std::vector<int4> ul;
             std::vector<int> ub;
-            build_umma_ranges(T.ker_v_f.data(), groups.data(), c->n_groups, c->NA, c->umma_nt, c->umma_bk,
-                              c->umma_ntiles, ul, ub);
+            build_umma_ranges(ranges.data(), c->n_groups, c->umma_nt, nk, c->umma_ntiles, ul, ub);
             void *dl = nullptr, *dbg = nullptr;
             if ((s = dalloc(c, &dl, std::max<size_t>(16, ul.size() * sizeof(int4)))) != BFPN_OK) return s;
             c->ulist = static_cast<int4*>(dl);
