@@ -299,7 +299,7 @@ void choose_plane_transport(bfpn_ctx* c) {
 // whole-plane kernel (or any supported one, option 2), in both precisions and
 // for any directions, unless an option names another kernel for the plane.
 bool march_transport(const bfpn_ctx* c) {
-    if (!c->tr_pairs || c->tr_stream == 0 || !transport_march_supported(c->Ny)) return false;
+    if (!c->tr_pairs || c->tr_stream == 0 || !transport_march_supported(c->Ny, c->NA)) return false;
     if (c->tr_stream == 2) return c->tr_stream_ok && c->tr_pairs_ok;
     if (c->tr_plane) return false;
     return (c->tr_stream_ok && c->tr_pairs_ok) || !c->tr_named;

@@ -308,7 +308,7 @@ bool transport_cluster_supported(int Ny, int Nz);
 template <typename T> cudaError_t launch_transport_march(const TransportArgs<T>& a, int lines, cudaStream_t s);
 cudaError_t launch_transport_march_slots(const TransportArgs<float>* args, const int* begin, int nslots, int blocks,
                                          int Ny, int NA, int lines, cudaStream_t s);
-bool transport_march_supported(int Ny);
+bool transport_march_supported(int Ny, int NA);
 int transport_march_chunks(int NA, size_t elem);
 int transport_march_lines(const double* omega, int NA, size_t elem);
 // Any plane, in 27 x 27 output tiles with a 4-cell halo, out of place;

@@ -29,11 +29,11 @@
 // each).  Measured per launch on a B200 (float; before: the row-streaming kernel
 // with its y-stencil in shared memory, or, for directions that do not pair and
 // for FP64, 27 x 27 tiles with halos and one angle per thread):
-//   81 x 81 x 400 angles x 500 groups     5.72  -> 4.14 ms (issue 70 % busy)
-//   49 x 49 x 256 x 400                   1.17  -> 0.98 ms
-//   38 x 30 x (15 x 12) x 301, unpaired   1.38  -> 0.42 ms
-//   62 x 62 x (7 x 15) x 94, unpaired     0.86  -> 0.39 ms
-//   FP64 31 x 47 x (14 x 16) x 42         0.747 -> 0.169 ms
+//   81 x 81 x 400 angles x 500 groups     5.72  -> 3.93 ms (issue 70 % busy)
+//   49 x 49 x 256 x 400                   1.17  -> 0.94 ms
+//   38 x 30 x (15 x 12) x 301, unpaired   1.38  -> 0.39 ms
+//   62 x 62 x (7 x 15) x 94, unpaired     0.86  -> 0.32 ms
+//   FP64 31 x 47 x (14 x 16) x 42         0.747 -> 0.155 ms
 #include "common.cuh"
 #include "async_copy.cuh"
 
@@ -50,7 +50,8 @@ constexpr int kMarchPitch = 48;   // bytes per position in shared memory: the ch
 constexpr int kMarchChunk = 32;   // bytes of consecutive angles per block
 
 // ---- arithmetic of one line value: a pair of float angles, or one double ----
-__device__ __forceinline__ float2 vsub(float2 x, float2 y) { return __ffma2_rn(y, make_float2(-1.f, -1.f), x); }
+__device__ __forceinline__ float2 vneg(float2 x) { return make_float2(-x.x, -x.y); }  // (a modifier of the operand)
+__device__ __forceinline__ float2 vsub(float2 x, float2 y) { return __fadd2_rn(x, vneg(y)); }
 __device__ __forceinline__ float2 vadd(float2 x, float2 y) { return __fadd2_rn(x, y); }
 __device__ __forceinline__ float2 vmul(float2 x, float2 y) { return __fmul2_rn(x, y); }
 __device__ __forceinline__ float2 vfma(float2 x, float2 y, float2 z) { return __ffma2_rn(x, y, z); }
@@ -192,14 +193,14 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
     constexpr int NP = 2;
     const bool vec = rc.lg == 1;
     int so[NP];        // shared-memory byte offset in a row
-    size_t go[NP];     // global byte offset in a row
+    unsigned go[NP];   // global byte offset in a row
     bool in[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
         const int v = tid + k * static_cast<int>(blockDim.x), q = v >> 1, o = (v & 1) * 16;
         in[k] = v < 2 * Ny1 && o < rc.valid;
         so[k] = q * kMarchPitch + o;
-        go[k] = static_cast<size_t>(q) * abytes + o;
+        go[k] = static_cast<unsigned>(q * abytes + o);
     }
     auto fill = [&](int r) {  // row r into slot r % RF; one commit group per call
         if (r <= Nz) {
@@ -258,18 +259,26 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
     const bool lone = LONE && e1 == e0;
     const int at0 = e0 & ~(W - 1);
     const bool dny = omega(e0, 0) < T(0), dnz = omega(e0, 1) < T(0);
-    V wy, wz;  // |omega_y| / dy (the line runs downwind), omega_z / dz
+    // -dt/2 |omega_y| / dy (the line runs downwind) and -dt/2 omega_z / dz: what a
+    // difference of two fluxes adds to a cell in half a step
+    V wy, wz;
+    // Where registers are scarcest, z fluxes are kept doubled: the slope's half and sign
+    // then need none (81 x 81 3.22 -> 3.15 ms per 400 groups, 62 x 62 unpaired 0.348 ->
+    // 0.318; paired lines of two cells lose, 49 x 49 0.941 -> 0.982, and so does FP64,
+    // 81 x 81 0.993 -> 1.010).
+    constexpr bool kDouble = W == 2 && (YT >= 3 || LONE);
+    const T hdt = T(-0.5) * a.dt, hdz = (kDouble ? T(-0.25) : T(-0.5)) * a.dt;
     if constexpr (W == 2) {
-        wy = make_float2(fabsf(omega(at0, 0) / a.dy), fabsf(omega(at0 + 1, 0) / a.dy));
-        wz = make_float2(omega(at0, 1) / a.dz, omega(at0 + 1, 1) / a.dz);
+        wy = make_float2(hdt * fabsf(omega(at0, 0) / a.dy), hdt * fabsf(omega(at0 + 1, 0) / a.dy));
+        wz = make_float2(hdz * (omega(at0, 1) / a.dz), hdz * (omega(at0 + 1, 1) / a.dz));
     } else {
-        wy = fabs(omega(e0, 0) / a.dy);
-        wz = omega(e0, 1) / a.dz;
+        wy = hdt * fabs(omega(e0, 0) / a.dy);
+        wz = hdz * (omega(e0, 1) / a.dz);
     }
-    const V hz = LineOf<T>::both(dnz ? T(-0.5) : T(0.5));
+    const V hz = LineOf<T>::both((dnz ? T(-1) : T(1)) * (kDouble ? T(1) : T(0.5)));
     // half the slope, kept where the difference towards higher y is at least eps
     const V hl = LineOf<T>::both(dny ? T(0.5) : T(0)), hr = LineOf<T>::both(dny ? T(0) : T(0.5));
-    const V ndt = LineOf<T>::both(-a.dt), nhdt = LineOf<T>::both(T(-0.5) * a.dt);
+    const V two = LineOf<T>::both(T(2));
     const T lo = a.preserve_sign ? -INFINITY : T(0);
 
     // ---- this thread's cells: positions YT sl + c - pad along the line ----
@@ -285,7 +294,7 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
     }
     auto load = [&](const T* row, int c) -> V { return *reinterpret_cast<const V*>(row + at[c]); };
 
-    // y-divergence (times |w| / dy) of the row x held by the line's lanes
+    // flux differences along y of the row x held by the line's lanes
     auto y_div = [&](const V (&x)[YT], V (&dy)[YT]) {
         V d[YT + 1], d2[YT + 1], k[YT + 1], g[YT];
         d[0] = vmul(vsub(x[0], lane_up(x[YT - 1], LW)), mL);
@@ -300,14 +309,21 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
 #pragma unroll
         for (int c = 0; c < YT; ++c)
             g[c] = vfma(march_limit(d[c], d2[c], d[c + 1], d2[c + 1]), vfma(k[c], hl, vmul(k[c + 1], hr)), x[c]);
-        dy[0] = vmul(wy, vmul(vsub(g[0], lane_up(g[YT - 1], LW)), mL));
+        dy[0] = vmul(vsub(g[0], lane_up(g[YT - 1], LW)), mL);
 #pragma unroll
-        for (int c = 1; c < YT; ++c) dy[c] = vmul(wy, vsub(g[c], g[c - 1]));
+        for (int c = 1; c < YT; ++c) dy[c] = vsub(g[c], g[c - 1]);
     };
     // z face of the cell with value x between the differences back and fwd
-    auto z_face = [&](V back, V fwd, V x) {
-        return vfma(march_limit(back, vadd(back, back), fwd, vadd(fwd, fwd)), vmul(march_keep(fwd), hz), x);
+    auto z_face = [&](auto DNZc, V back, V fwd, V x) {
+        if constexpr (kDouble) {
+            constexpr int DNZ = decltype(DNZc)::value;
+            const V k = march_keep(fwd), m = march_limit(back, vadd(back, back), fwd, vadd(fwd, fwd));
+            return vfma(m, DNZ == 0 ? k : DNZ == 1 ? vneg(k) : vmul(k, hz), vadd(x, x));
+        } else {
+            return vfma(march_limit(back, vadd(back, back), fwd, vadd(fwd, fwd)), vmul(march_keep(fwd), hz), x);
+        }
     };
+    auto z_flat = [&](V x) { return kDouble ? vadd(x, x) : x; };  // the face of a cell without slope
 
     // Row r has landed, the rows of iteration r-1 are written and may leave.
     auto meet = [&](int r) {
@@ -325,7 +341,8 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
         meet(0);
 #pragma unroll
         for (int c = 0; c < YT; ++c) {
-            f1[c] = f2[c] = g1[c] = p1[c] = gp[c] = load(ring, c);
+            f1[c] = f2[c] = p1[c] = load(ring, c);
+            g1[c] = gp[c] = z_flat(f1[c]);
             zd[c] = ez[c] = pd[c] = ep[c] = t1[c] = t2[c] = zero;
         }
         // one copy of the body for every row: the march is long straight-line code
@@ -342,9 +359,9 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
                 for (int c = 0; c < YT; ++c) {
                     x[c] = load(row, c);
                     const V d = vsub(x[c], f1[c]);
-                    const V g = z_face(zd[c], d, f1[c]);
+                    const V g = z_face(DNZc, zd[c], d, f1[c]);
                     const V e = vsub(g, g1[c]);
-                    dz[c] = vmul(wz, DNZ == 2 ? vselect(dnz, e, ez[c]) : e);
+                    dz[c] = DNZ == 2 ? vselect(dnz, e, ez[c]) : e;
                     if (DNZ == 2) ez[c] = e;
                     g1[c] = g;
                     zd[c] = d;
@@ -353,14 +370,14 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
                 y_div(fi, dy);
 #pragma unroll
                 for (int c = 0; c < YT; ++c) {
-                    const V d = vadd(dy[c], dz[c]);
-                    p[c] = vmax(vfma(ndt, d, fi[c]), lo);
-                    t[c] = vfma(nhdt, d, fi[c]);
+                    const V d = vfma(wy, dy[c], vmul(wz, dz[c]));
+                    p[c] = vmax(vfma(two, d, fi[c]), lo);
+                    t[c] = vadd(fi[c], d);
                 }
                 y_div(p, dy);
 #pragma unroll
                 for (int c = 0; c < YT; ++c) {
-                    t[c] = vfma(nhdt, dy[c], t[c]);
+                    t[c] = vfma(wy, dy[c], t[c]);
                     if (LAG == 2) f2[c] = f1[c];
                     f1[c] = x[c];
                 }
@@ -375,7 +392,8 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
 #pragma unroll
                 for (int c = 0; c < YT; ++c) {
                     pd[c] = ep[c] = zero;
-                    gp[c] = p1[c] = p[c];
+                    p1[c] = p[c];
+                    gp[c] = z_flat(p[c]);
                     if (LAG == 2) t2[c] = t1[c];
                     t1[c] = t[c];
                 }
@@ -385,10 +403,10 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
 #pragma unroll
             for (int c = 0; c < YT; ++c) {
                 const V d = vsub(p[c], p1[c]);
-                const V g = z_face(pd[c], d, p1[c]);
+                const V g = z_face(DNZc, pd[c], d, p1[c]);
                 const V e = vsub(g, gp[c]);
-                const V dz = vmul(wz, DNZ == 2 ? vselect(dnz, e, ep[c]) : e);
-                const V v = vmax(vfma(nhdt, dz, LAG == 1 ? t1[c] : t2[c]), lo);
+                const V dz = DNZ == 2 ? vselect(dnz, e, ep[c]) : e;
+                const V v = vmax(vfma(wz, dz, LAG == 1 ? t1[c] : t2[c]), lo);
                 // (a row before the first lands in a slot that a later row takes)
                 if constexpr (!LONE) {
                     store_if(reinterpret_cast<V*>(out + at[c]), v, own[c]);
@@ -469,7 +487,8 @@ cudaError_t with_shape(const MarchShape& m, const F& f) {
 
 }  // namespace
 
-bool transport_march_supported(int Ny) { return Ny >= 1 && Ny + 1 <= 128; }
+// (a row's byte offsets stay within 32 bits)
+bool transport_march_supported(int Ny, int NA) { return Ny >= 1 && Ny + 1 <= 128 && NA <= 1 << 20; }
 
 int transport_march_chunks(int NA, size_t elem) {
     const int ac = kMarchChunk / static_cast<int>(elem);
@@ -494,7 +513,7 @@ int transport_march_lines(const double* omega, int NA, size_t elem) {
 
 template <typename T>
 cudaError_t launch_transport_march(const TransportArgs<T>& a, int lines, cudaStream_t s) {
-    if (!transport_march_supported(a.Ny) || lines <= 0) return cudaErrorNotSupported;
+    if (!transport_march_supported(a.Ny, a.NA) || lines <= 0) return cudaErrorNotSupported;
     const MarchShape m = march_shape(a.Ny + 1);
     const int n_chunks = transport_march_chunks(a.NA, sizeof(T));
     const long long blocks = static_cast<long long>(a.Ng) * n_chunks;
@@ -517,7 +536,7 @@ template cudaError_t launch_transport_march<double>(const TransportArgs<double>&
 cudaError_t launch_transport_march_slots(const TransportArgs<float>* args, const int* begin, int nslots, int blocks,
                                          int Ny, int NA, int lines, cudaStream_t s) {
     if (nslots <= 0 || blocks <= 0) return cudaSuccess;
-    if (!transport_march_supported(Ny) || lines <= 0) return cudaErrorNotSupported;
+    if (!transport_march_supported(Ny, NA) || lines <= 0) return cudaErrorNotSupported;
     const MarchShape m = march_shape(Ny + 1);
     const int n_chunks = transport_march_chunks(NA, 4);
     return with_shape(m, [&](auto lw, auto yt) {
