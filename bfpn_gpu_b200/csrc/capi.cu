@@ -340,13 +340,32 @@ void convert_values(T* dev_side, double* host, size_t n, bool up) {
     }
 }
 
+// Pinned memory of the context, allocated on first use and allowed while another
+// thread captures a graph; false (no error left behind) where there is none to be
+// had: the caller then takes its path through pageable memory.
+bool host_buffer(bfpn_ctx* c, void*& p, size_t bytes, unsigned flags) {
+    if (p) return true;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaHostAlloc(&p, bytes, flags);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+        return false;
+    }
+    c->host_allocs.push_back(p);
+    return true;
+}
+
+bool stage_ready(bfpn_ctx* c) {
+    return host_buffer(c, c->stage[0], kStageBytes, cudaHostAllocDefault) &&
+           host_buffer(c, c->stage[1], kStageBytes, cudaHostAllocDefault);
+}
+
+// (stage_ready came first)
 template <typename T>
 bfpn_status staged_transfer(bfpn_ctx* c, void* dev, double* host, size_t n, bool up) {
-    for (void*& b : c->stage)
-        if (!b) {
-            CUDA_TRY(c, cudaHostAlloc(&b, kStageBytes, cudaHostAllocDefault));
-            c->host_allocs.push_back(b);
-        }
     const size_t chunk = kStageBytes / sizeof(T), chunks = (n + chunk - 1) / chunk;
     // workers take an equal part of every chunk; the caller's thread moves the chunks
     std::atomic<size_t> ready{0};        // chunks the workers may take
@@ -409,7 +428,8 @@ bfpn_status staged_transfer(bfpn_ctx* c, void* dev, double* host, size_t n, bool
 
 template <typename T>
 bfpn_status upload_as(bfpn_ctx* c, void* dst, const double* host, size_t n) {
-    if (n * sizeof(T) > kStageSmall) return staged_transfer<T>(c, dst, const_cast<double*>(host), n, true);
+    if (n * sizeof(T) > kStageSmall && stage_ready(c))
+        return staged_transfer<T>(c, dst, const_cast<double*>(host), n, true);
     if (sizeof(T) == sizeof(double)) {
         CUDA_TRY(c, cudaMemcpyAsync(dst, host, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
         return BFPN_OK;
@@ -1288,7 +1308,8 @@ bfpn_status run_steps(bfpn_ctx* c, int nsteps) {
 
 template <typename T>
 bfpn_status download_as(bfpn_ctx* c, const void* dev, double* host, size_t n) {
-    if (n * sizeof(T) > kStageSmall) return staged_transfer<T>(c, const_cast<void*>(dev), host, n, false);
+    if (n * sizeof(T) > kStageSmall && stage_ready(c))
+        return staged_transfer<T>(c, const_cast<void*>(dev), host, n, false);
     if (sizeof(T) == sizeof(double)) {
         CUDA_TRY(c, cudaMemcpyAsync(host, dev, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
@@ -1324,13 +1345,8 @@ struct StepExport {
     int err;
 };
 
+// (its buffer, c->step_export, is there)
 bfpn_status export_history(bfpn_ctx* c, int first, int count, double* idd_out, double* proxy_out, bool* clean) {
-    if (!c->step_export) {
-        void* h = nullptr;
-        CUDA_TRY(c, cudaHostAlloc(&h, sizeof(StepExport), cudaHostAllocMapped));
-        c->host_allocs.push_back(h);
-        c->step_export = h;
-    }
     auto* h = static_cast<StepExport*>(c->step_export);
     void* d = nullptr;
     CUDA_TRY(c, cudaHostGetDevicePointer(&d, h, 0));
@@ -1889,7 +1905,7 @@ bfpn_status bfpn_step(bfpn_ctx* c, int32_t nsteps, double* idd_out, double* prox
     const int first = c->steps_done;
     bfpn_status s = bfpn_step_async(c, nsteps);
     if (s != BFPN_OK) return s;
-    if (nsteps > 0 && nsteps <= kExportSteps) {
+    if (nsteps > 0 && nsteps <= kExportSteps && host_buffer(c, c->step_export, sizeof(StepExport), cudaHostAllocMapped)) {
         bool clean = false;
         if ((s = export_history(c, first, nsteps, idd_out, proxy_out, &clean)) != BFPN_OK) return s;
         CUDA_TRY(c, collect_profile(c));

@@ -169,3 +169,61 @@ def test_caller_owned_dose_shapes(ny, nz, nmu, nom, ng, shift, dtype, precision)
         want = [float(((k[:, 0] * psi1 + k[:, 1] * psi2) * pos).sum()) * vol, float(f0.sum()) * g.Lg / ng]
         # sums of at most 2e7 positive terms in double: 1e-11 covers any order
         assert np.allclose(out.cpu().numpy(), want, rtol=1e-11, atol=0.0)
+
+
+# 48 positions and 16-column remainders of the tensor-core output tile, odd angle
+# counts, one position tile exactly, one more and one less; bars as for the same
+# operator in test_parity_gpu.py
+@pytest.mark.parametrize("ny,nz,nmu,nom", [(7, 5, 6, 8), (8, 6, 7, 9), (7, 7, 4, 4), (12, 4, 11, 3), (6, 8, 16, 17)])
+def test_tensor_core_source_shapes(ny, nz, nmu, nom):
+    cfg = small_cfg(ny=ny, nz=nz, nmu=nmu, nom=nom)
+    ctx, ora = build(cfg, precision=capi.PREC_MIXED)
+    set_both(ctx, ora, _states(ctx, 45, capi.PREC_MIXED))
+    s = ora.source()
+    ctx.secondary_source()
+    assert np.abs(s).max() > 0
+    assert rel_err(ctx.source(), s) < 2e-5
+
+
+# below the staging size, just above it, a partial last chunk, an odd count
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("ny,nz,nmu,nom,ng", [(15, 15, 8, 8, 128), (15, 16, 8, 16, 65), (16, 16, 16, 16, 40),
+                                              (26, 24, 7, 9, 101)])
+def test_state_transfer_round_trip(ny, nz, nmu, nom, ng, precision):
+    """Values that both precisions hold come back as they went in."""
+    cfg = small_cfg(ny=ny, nz=nz, nmu=nmu, nom=nom, ng=ng, lg=1.475 * ng, beam_energy=1.0 * ng)
+    ctx, _ = build(cfg, precision=precision)
+    n = int(np.prod(ctx.shape))
+    a = (np.arange(n) % 65521).astype(np.float64) * 2.0 ** -20
+    b = -a[::-1].copy()
+    ctx.set_state(0, 0, a)
+    ctx.set_state(1, 1, b)
+    ctx.set_state(0, 0, b)
+    assert np.array_equal(ctx.get_state(1, 1), b)
+    assert np.array_equal(ctx.get_state(0, 0), b)
+
+
+@pytest.mark.parametrize("n", [255, 256, 257])
+def test_step_call_lengths(n):
+    """Results of one call around the most steps one export holds, against the
+    history of single steps bit for bit (the lite step has no fused forms)."""
+    cfg = small_cfg(ny=3, nz=3, nmu=3, nom=3, nx=300, lite_memory=True)
+    one, _ = build(cfg)
+    idd, prox = one.step(n)
+    many, _ = build(cfg)
+    got = [many.step(1) for _ in range(n)]
+    assert len(idd) == n and np.array_equal(idd, np.concatenate([g[0] for g in got]))
+    assert np.array_equal(prox, np.concatenate([g[1] for g in got]))
+    assert np.array_equal(one.get_state(0, 0), many.get_state(0, 0))
+
+
+# the default chunk of the whole-plane kernel changes at 33 points (16, 8 angles)
+@pytest.mark.parametrize("ny,nmu,nom", [(20, 5, 4), (24, 3, 6), (32, 5, 4)])
+def test_plane_transport_default_chunk(ny, nmu, nom):
+    cfg = small_cfg(ny=ny, nz=ny, nmu=nmu, nom=nom, ng=7, lg=1.475 * 7, beam_energy=7.0)
+    ctx, ora = build(cfg, precision=capi.PREC_MIXED)
+    set_both(ctx, ora, _states(ctx, 46, capi.PREC_MIXED))
+    for sp, cf in ((0, 0), (1, 1)):
+        ctx.transport(sp, cf, 0.5 * cfg.dt(), cf == 1)
+        ora.transport(sp, cf, 0.5 * cfg.dt(), cf == 1)
+    assert_states(ctx, ora, 2e-6)
