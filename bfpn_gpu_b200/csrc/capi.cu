@@ -1758,13 +1758,20 @@ bfpn_status bfpn_load_tables(bfpn_ctx* c, const double* mu, int32_t mu_rows, con
         {
             const int nk = (c->NA + c->umma_bk - 1) / c->umma_bk;
             std::vector<int2> ranges(static_cast<size_t>(c->n_groups) * c->umma_ntiles * nk);
-            void* dr = nullptr;
-            if ((s = dalloc(c, &dr, ranges.size() * sizeof(int2))) != BFPN_OK) return s;
+            // (the source's work buffer takes them where it is large enough: freeing
+            // an allocation would wait for every other beam on the device)
+            const size_t range_bytes = ranges.size() * sizeof(int2);
+            void *own = nullptr, *dr = c->A1;
+            if (!dr || c->a_bytes < range_bytes) {
+                if ((s = dalloc(c, &own, range_bytes)) != BFPN_OK) return s;
+                dr = own;
+            }
             CUDA_TRY(c, launch_angular_ranges(as<const float>(c->ker_v), c->groups, c->n_groups, c->NA, c->umma_nt, c->umma_bk,
                                               c->umma_ntiles, static_cast<int2*>(dr), c->stream));
-            CUDA_TRY(c, cudaMemcpyAsync(ranges.data(), dr, ranges.size() * sizeof(int2), cudaMemcpyDeviceToHost, c->stream));
+            CUDA_TRY(c, cudaMemcpyAsync(ranges.data(), dr, range_bytes, cudaMemcpyDeviceToHost, c->stream));
+            if (!own) CUDA_TRY(c, cudaMemsetAsync(dr, 0, range_bytes, c->stream));  // as the source expects it
             CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-            dfree(c, dr);
+            dfree(c, own);
             std::vector<int4> ul;
             std::vector<int> ub;
             build_umma_ranges(ranges.data(), c->n_groups, c->umma_nt, nk, c->umma_ntiles, ul, ub);

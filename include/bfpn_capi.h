@@ -255,10 +255,13 @@ int32_t bfpn_source_groups(bfpn_ctx* ctx);
  * BFPN_OPT_CUDA_GRAPHS: 1 (default) replays each depth step as a CUDA graph.
  * BFPN_OPT_PLANE_TRANSPORT: 1 (default) runs the transport with the unrolled
  *   kernels: one block per whole plane for square planes with
- *   Ny = Nz in {4,6,8,10,12,14,16,20,24,32}, 27 x 27 tiles for planes too large
- *   for one block; 0 uses the general line-walk kernel; a larger value selects
- *   the angles per block (whole planes: 8 or 16 mixed, 4 or 8 FP64; tiles: 4 or
- *   8 mixed, 2 or 4 FP64).  All compute the same values.
+ *   Ny = Nz in {4,6,8,10,12,14,16,20,24,32}, the marching kernel (see
+ *   BFPN_OPT_STREAM_TRANSPORT) or 27 x 27 tiles for the others; 0 uses the
+ *   general line-walk kernel; a larger value selects the angles per block
+ *   (whole planes: 8 or 16 mixed -- by default 16 up to 21 points, then 8 --,
+ *   4 or 8 FP64; tiles, which it then also selects where directions do not
+ *   pair and in FP64: 4 or 8 mixed, 2 or 4 FP64).  All compute the same values
+ *   (the marching kernel to rounding).
  * BFPN_OPT_PAIRED_ANGLES: 1 (default) lets mixed-precision kernels carry
  *   two lines per thread on packed fp32x2 arithmetic: the whole-plane
  *   transport two angles (when NA is even and the angles of each pair
@@ -270,8 +273,9 @@ int32_t bfpn_source_groups(bfpn_ctx* ctx);
  *   thread-block clusters: 2 to 8 CTAs hold one plane in their shared memory
  *   and exchange edge rows through distributed shared memory, in place;
  *   2 also uses it for Ny = Nz = 20 (in place of the whole-plane kernel);
- *   0 leaves those planes to the tiled kernel.  Values agree with the other
- *   kernels to float rounding.
+ *   0 leaves those planes to the tiled kernel.  It runs where
+ *   BFPN_OPT_STREAM_TRANSPORT is 0.  Values agree with the other kernels to
+ *   float rounding.
  * BFPN_OPT_LANE_CHUNK / BFPN_OPT_ENERGY_CHUNK (out-of-core mode only): lanes
  *   per lane chunk (rounded down to whole positions, at least one; default
  *   262,144, the reference's --lane-chunk) and groups per group chunk (default
@@ -282,18 +286,19 @@ int32_t bfpn_source_groups(bfpn_ctx* ctx);
  *   inside one CUDA graph, and within each half runs the transport-angle-
  *   transport chain of psi^2 beside that of psi^1; 1 overlaps the halves
  *   only; 0 runs everything one kernel after the other.  Applies when graphs
- *   are on and the transport is in place (whole-plane or cluster kernels);
+ *   are on and the transport is in place (all but the tiled and some line-walk forms);
  *   every bfpn_step / bfpn_step_async call still ends on whole steps.  Same
  *   kernels on the same inputs: the same values.
- * BFPN_OPT_STREAM_TRANSPORT: 1 (default) runs the mixed-precision transport
- *   of planes without a whole-plane kernel (Ny + 1 <= 256, any Nz, paired
- *   angles) with the row-streaming kernel: one block per (group, 8-angle)
- *   plane walks the z rows, the z-stencil in registers and one row of the
- *   y-stencil in shared memory, in place; 2 also uses it where a whole-plane
- *   kernel exists; 0 leaves those planes to the cluster / tiled kernels.
- *   Same values as the whole-plane kernel.
+ * BFPN_OPT_STREAM_TRANSPORT: 1 (default) runs the transport of planes without
+ *   a whole-plane kernel by walking the z rows, in place: up to Ny + 1 = 128 the
+ *   marching kernel (both precisions, any directions, any Nz: whole y lines in
+ *   the lanes of a warp, the z-stencil in registers, neighbours by shuffles), up
+ *   to 256 the row-streaming kernel (mixed precision, paired angles); 2 also
+ *   uses them where a whole-plane kernel exists (mixed precision, paired
+ *   angles); 0 leaves those planes to the cluster / tiled kernels.  Values agree
+ *   with the whole-plane kernel to rounding.
  * BFPN_OPT_FUSED_ENERGY: 1 (default) runs, in mixed precision with step
- *   overlap on (eq15 energy, NA a multiple of 4, the tensor-core source), the
+ *   overlap on (eq15 energy, the tensor-core source), the
  *   primary's closing energy half-step of each step and the opening half-step
  *   of the next as one kernel, which also writes the source's split-bf16
  *   operand: per step one primary energy pass and the operand's pack pass
@@ -418,8 +423,10 @@ bfpn_status bfpn_batch_run(const bfpn_beam* beams, int32_t n, const int32_t* dev
  * tables, beam, depth-step count and IDD history, and join or leave at any
  * step (continuous batching).  The step of the current slot set is one CUDA
  * graph.  Kernel variants (angles per transport block, DST ring stages,
- * energy kernel form) are timed per shape class on the bundle's first steps
- * and the fastest kept for the process (autotuning); all variants compute the
+ * lanes per energy thread) are timed per shape class on six of the bundle's
+ * steps, the first four of which only load the kernels (beams with fewer steps
+ * left run the defaults), and the fastest kept for the process (autotuning);
+ * all variants compute the
  * same states.  Each beam's IDD history equals its single-context run up to
  * the order of the IDD partial sums. */
 typedef struct bfpn_bundle bfpn_bundle;
@@ -428,7 +435,7 @@ enum {
     BFPN_BUNDLE_OPT_AUTOTUNE = 1,          /* 1 (default) tune on first use, 0 use the defaults / settings below */
     BFPN_BUNDLE_OPT_TRANSPORT_ANGLES = 2,  /* 8 or 16 angles per whole-plane transport block (turns tuning off) */
     BFPN_BUNDLE_OPT_DST_STAGES = 3,        /* 2 or 3 DST ring stages (turns tuning off) */
-    BFPN_BUNDLE_OPT_ENERGY_RING = 4        /* 1 ring energy kernel, 0 register kernel (turns tuning off) */
+    BFPN_BUNDLE_OPT_ENERGY_RING = 4        /* 1: four lanes per energy thread, 0: one (turns tuning off) */
 };
 
 /* BFPN_OK when a bundle can hold the beam (host-side check of its precision,

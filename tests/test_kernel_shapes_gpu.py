@@ -13,6 +13,7 @@ import pytest
 
 from conftest import rel_err
 from test_parity_gpu import OP_TOL, STEP_TOL, assert_states, build, seeded_states, set_both, small_cfg
+from test_bundle_gpu import alone, check, pick
 from bfpn_gpu_b200 import capi
 
 pytestmark = pytest.mark.gpu
@@ -227,3 +228,17 @@ def test_plane_transport_default_chunk(ny, nmu, nom):
         ctx.transport(sp, cf, 0.5 * cfg.dt(), cf == 1)
         ora.transport(sp, cf, 0.5 * cfg.dt(), cf == 1)
     assert_states(ctx, ora, 2e-6)
+
+
+# one step too short for a tuning run, exactly one, one longer (bars of test_bundle_gpu.py)
+@pytest.mark.parametrize("n", [5, 6, 7])
+def test_bundle_tuning_lengths(n):
+    reqs = pick(16, 12, 2, n)
+    refs = [alone(r) for r in reqs]
+    with capi.Bundle(max_slots=2) as b:
+        slots = [b.admit(r.beam()) for r in reqs]
+        b.step(1000)
+        b.sync()
+        assert b.running() == 0
+        for s, ref in zip(slots, refs):
+            check(b.collect(s), ref)
