@@ -296,13 +296,18 @@ void choose_plane_transport(bfpn_ctx* c) {
 }
 
 // The marching kernel runs this context's transport: planes without a
-// whole-plane kernel (or any supported one, option 2), in both precisions and
-// for any directions, unless an option names another kernel for the plane.
+// whole-plane kernel (or any supported one, option 2), unless an option names
+// another kernel for the plane; of float planes whose directions do not pair,
+// those of several line-walk tiles.
 bool march_transport(const bfpn_ctx* c) {
     if (!c->tr_pairs || c->tr_stream == 0 || !transport_march_supported(c->Ny, c->NA)) return false;
     if (c->tr_stream == 2) return c->tr_stream_ok && c->tr_pairs_ok;
     if (c->tr_plane) return false;
-    return (c->tr_stream_ok && c->tr_pairs_ok) || !c->tr_named;
+    if (c->tr_stream_ok && c->tr_pairs_ok) return true;
+    // float directions that do not pair: planes of several line-walk tiles, whose
+    // unrolled tiled kernel the march equals value for value (smaller ones keep the
+    // line walks, whose order of rounding it does not have)
+    return !c->tr_named && (c->elem == 8 || !c->tr_inplace);
 }
 
 // The row-streaming kernel runs this context's transport (it needs paired

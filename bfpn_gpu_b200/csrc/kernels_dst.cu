@@ -5,9 +5,9 @@
 // One block holds a tile of consecutive slices in shared memory and runs the
 // forward u, forward v * factor * inverse v and inverse u passes there, a thread
 // carrying a whole line in registers -- two lines on fp32x2 arithmetic for float
-// state -- so a line's N ceil(N/2) products take no shared-memory traffic (the
+// state -- so a line's products take no shared-memory traffic (the
 // run-time-length kernel reads two operands per product: 15 x 12 angles took
-// 1.36 ms for 62M float cells, 0.26 here).  The transforms are compiled per length and
+// 1.36 ms for 62M float cells, 0.29 here).  The transforms are compiled per length and
 // picked by a block-uniform switch; a kernel is compiled for lengths up to 8,
 // 16, 24 and 32, since the longest sets its registers.  What bounds it: the fma
 // pipe and, between the passes, the block's barriers, which the other blocks of
@@ -34,8 +34,23 @@ template <> struct RectLine<double> {
     using V = double;
     static constexpr int W = 1;
 };
+// Float: the N x N products in order, the run-time-length kernel's sums bit for bit
+// (folding the line first would halve them, but round differently).
 template <int N>
-__device__ __forceinline__ void rect_dst(const float (&c)[(N + 1) / 2], const float2 (&x)[N], float2 (&y)[N]) { dst1_pair<N>(c, x, y); }
+__device__ __forceinline__ void rect_dst(const float (&c)[(N + 1) / 2], const float2 (&x)[N], float2 (&y)[N]) {
+#pragma unroll
+    for (int m = 0; m < N; ++m) {
+        float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int k = sine_k(N, m, i);
+            if (k == 0) continue;
+            const float cc = sine_neg(N, m, i) ? -c[k - 1] : c[k - 1];
+            acc = __ffma2_rn(make_float2(cc, cc), x[i], acc);
+        }
+        y[m] = acc;
+    }
+}
 template <int N>
 __device__ __forceinline__ void rect_dst(const double (&c)[(N + 1) / 2], const double (&x)[N], double (&y)[N]) { dst1<N, double>(c, x, y); }
 

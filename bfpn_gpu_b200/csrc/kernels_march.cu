@@ -29,11 +29,11 @@
 // each).  Measured per launch on a B200 (float; before: the row-streaming kernel
 // with its y-stencil in shared memory, or, for directions that do not pair and
 // for FP64, 27 x 27 tiles with halos and one angle per thread):
-//   81 x 81 x 400 angles x 500 groups     5.72  -> 3.93 ms (issue 70 % busy)
-//   49 x 49 x 256 x 400                   1.17  -> 0.94 ms
-//   38 x 30 x (15 x 12) x 301, unpaired   1.38  -> 0.39 ms
+//   81 x 81 x 400 angles x 500 groups     5.72  -> 4.00 ms (issue 70 % busy)
+//   49 x 49 x 256 x 400                   1.17  -> 0.96 ms
+//   38 x 30 x (15 x 12) x 301, unpaired   1.38  -> 0.42 ms
 //   62 x 62 x (7 x 15) x 94, unpaired     0.86  -> 0.32 ms
-//   FP64 31 x 47 x (14 x 16) x 42         0.747 -> 0.155 ms
+//   FP64 31 x 47 x (14 x 16) x 42         0.747 -> 0.158 ms
 #include "common.cuh"
 #include "async_copy.cuh"
 
@@ -259,26 +259,24 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
     const bool lone = LONE && e1 == e0;
     const int at0 = e0 & ~(W - 1);
     const bool dny = omega(e0, 0) < T(0), dnz = omega(e0, 1) < T(0);
-    // -dt/2 |omega_y| / dy (the line runs downwind) and -dt/2 omega_z / dz: what a
-    // difference of two fluxes adds to a cell in half a step
-    V wy, wz;
     // Where registers are scarcest, z fluxes are kept doubled: the slope's half and sign
     // then need none (81 x 81 3.22 -> 3.15 ms per 400 groups, 62 x 62 unpaired 0.348 ->
     // 0.318; paired lines of two cells lose, 49 x 49 0.941 -> 0.982, and so does FP64,
     // 81 x 81 0.993 -> 1.010).
     constexpr bool kDouble = W == 2 && (YT >= 3 || LONE);
-    const T hdt = T(-0.5) * a.dt, hdz = (kDouble ? T(-0.25) : T(-0.5)) * a.dt;
+    V wy, wz;  // |omega_y| / dy (the line runs downwind), omega_z / dz (half of it for doubled fluxes)
+    const T zs1 = kDouble ? T(0.5) : T(1);
     if constexpr (W == 2) {
-        wy = make_float2(hdt * fabsf(omega(at0, 0) / a.dy), hdt * fabsf(omega(at0 + 1, 0) / a.dy));
-        wz = make_float2(hdz * (omega(at0, 1) / a.dz), hdz * (omega(at0 + 1, 1) / a.dz));
+        wy = make_float2(fabsf(omega(at0, 0) / a.dy), fabsf(omega(at0 + 1, 0) / a.dy));
+        wz = make_float2(zs1 * (omega(at0, 1) / a.dz), zs1 * (omega(at0 + 1, 1) / a.dz));
     } else {
-        wy = hdt * fabs(omega(e0, 0) / a.dy);
-        wz = hdz * (omega(e0, 1) / a.dz);
+        wy = fabs(omega(e0, 0) / a.dy);
+        wz = zs1 * (omega(e0, 1) / a.dz);
     }
     const V hz = LineOf<T>::both((dnz ? T(-1) : T(1)) * (kDouble ? T(1) : T(0.5)));
     // half the slope, kept where the difference towards higher y is at least eps
     const V hl = LineOf<T>::both(dny ? T(0.5) : T(0)), hr = LineOf<T>::both(dny ? T(0) : T(0.5));
-    const V two = LineOf<T>::both(T(2));
+    const V ndt = LineOf<T>::both(-a.dt), nhdt = LineOf<T>::both(T(-0.5) * a.dt);
     const T lo = a.preserve_sign ? -INFINITY : T(0);
 
     // ---- this thread's cells: positions YT sl + c - pad along the line ----
@@ -294,7 +292,7 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
     }
     auto load = [&](const T* row, int c) -> V { return *reinterpret_cast<const V*>(row + at[c]); };
 
-    // flux differences along y of the row x held by the line's lanes
+    // y-divergence (times |w| / dy) of the row x held by the line's lanes
     auto y_div = [&](const V (&x)[YT], V (&dy)[YT]) {
         V d[YT + 1], d2[YT + 1], k[YT + 1], g[YT];
         d[0] = vmul(vsub(x[0], lane_up(x[YT - 1], LW)), mL);
@@ -309,9 +307,9 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
 #pragma unroll
         for (int c = 0; c < YT; ++c)
             g[c] = vfma(march_limit(d[c], d2[c], d[c + 1], d2[c + 1]), vfma(k[c], hl, vmul(k[c + 1], hr)), x[c]);
-        dy[0] = vmul(vsub(g[0], lane_up(g[YT - 1], LW)), mL);
+        dy[0] = vmul(wy, vmul(vsub(g[0], lane_up(g[YT - 1], LW)), mL));
 #pragma unroll
-        for (int c = 1; c < YT; ++c) dy[c] = vsub(g[c], g[c - 1]);
+        for (int c = 1; c < YT; ++c) dy[c] = vmul(wy, vsub(g[c], g[c - 1]));
     };
     // z face of the cell with value x between the differences back and fwd
     auto z_face = [&](auto DNZc, V back, V fwd, V x) {
@@ -370,14 +368,18 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
                 y_div(fi, dy);
 #pragma unroll
                 for (int c = 0; c < YT; ++c) {
-                    const V d = vfma(wy, dy[c], vmul(wz, dz[c]));
-                    p[c] = vmax(vfma(two, d, fi[c]), lo);
-                    t[c] = vadd(fi[c], d);
+                    // (rounded as in the kernels of these planes' other options, so the values
+                    // are theirs: the tiled kernel's sum is one fma, the paired kernels' two
+                    // operations; one scaled sum for p and t saved 2 % and differed by up to
+                    // 4e-5 in a sum of signed values)
+                    const V d = LONE || W == 1 ? vfma(wz, dz[c], dy[c]) : vadd(dy[c], vmul(wz, dz[c]));
+                    p[c] = vmax(vfma(ndt, d, fi[c]), lo);
+                    t[c] = vfma(nhdt, d, fi[c]);
                 }
                 y_div(p, dy);
 #pragma unroll
                 for (int c = 0; c < YT; ++c) {
-                    t[c] = vfma(wy, dy[c], t[c]);
+                    t[c] = vfma(nhdt, dy[c], t[c]);
                     if (LAG == 2) f2[c] = f1[c];
                     f1[c] = x[c];
                 }
@@ -406,7 +408,7 @@ __device__ __forceinline__ void march_body(const TransportArgs<T>& a, int n_chun
                 const V g = z_face(DNZc, pd[c], d, p1[c]);
                 const V e = vsub(g, gp[c]);
                 const V dz = DNZ == 2 ? vselect(dnz, e, ep[c]) : e;
-                const V v = vmax(vfma(wz, dz, LAG == 1 ? t1[c] : t2[c]), lo);
+                const V v = vmax(vfma(nhdt, vmul(wz, dz), LAG == 1 ? t1[c] : t2[c]), lo);
                 // (a row before the first lands in a slot that a later row takes)
                 if constexpr (!LONE) {
                     store_if(reinterpret_cast<V*>(out + at[c]), v, own[c]);

@@ -291,9 +291,10 @@ int32_t bfpn_source_groups(bfpn_ctx* ctx);
  *   kernels on the same inputs: the same values.
  * BFPN_OPT_STREAM_TRANSPORT: 1 (default) runs the transport of planes without
  *   a whole-plane kernel by walking the z rows, in place: up to Ny + 1 = 128 the
- *   marching kernel (both precisions, any directions, any Nz: whole y lines in
- *   the lanes of a warp, the z-stencil in registers, neighbours by shuffles), up
- *   to 256 the row-streaming kernel (mixed precision, paired angles); 2 also
+ *   marching kernel (both precisions, any Nz: whole y lines in the lanes of a
+ *   warp, the z-stencil in registers, neighbours by shuffles; float directions
+ *   that do not pair on planes of more than one line-walk tile, about 768
+ *   points), up to 256 the row-streaming kernel (mixed precision, paired angles); 2 also
  *   uses them where a whole-plane kernel exists (mixed precision, paired
  *   angles); 0 leaves those planes to the cluster / tiled kernels.  Values agree
  *   with the whole-plane kernel to rounding.

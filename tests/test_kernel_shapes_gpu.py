@@ -78,7 +78,10 @@ def test_fused_pass_shapes(shape, straggling):
 @pytest.mark.parametrize("ny,nz,ang", [(1, 3, (4, 4)), (2, 1, (5, 6)), (7, 9, (5, 3)), (8, 3, (4, 4)), (11, 2, (5, 6)),
                                        (23, 5, (5, 3)), (32, 4, (5, 6)), (37, 29, (4, 4)), (47, 2, (2, 2)),
                                        (48, 5, (5, 6)), (64, 3, (5, 3)), (80, 6, (5, 6)), (95, 2, (4, 4)),
-                                       (96, 3, (5, 6)), (127, 2, (5, 3))])
+                                       (96, 3, (5, 6)), (127, 2, (5, 3)),
+                                       # beyond one line-walk tile: float's lone angles march too
+                                       (7, 100, (5, 6)), (11, 70, (5, 3)), (27, 28, (3, 3)), (32, 24, (5, 6)),
+                                       (47, 17, (5, 3)), (64, 12, (5, 6)), (96, 8, (5, 3)), (127, 6, (5, 6))])
 def test_march_transport_shapes(ny, nz, ang, precision):
     cfg = small_cfg(ny=ny, nz=nz, nmu=ang[0], nom=ang[1], ng=3, ly=0.2 * ny, lz=0.25 * nz)
     ctx, ora = build(cfg, precision=precision)
