@@ -233,7 +233,7 @@ def kernel_bytes(cls, cells, elem, n_groups, nyz, NA, fused=False):
 # DRAM bytes (read + write) per cell of one launch of each kernel class, from ncu
 # captures of the same kernels on a smaller state of the same lateral and
 # angular grid (profiles/*.txt: the 20x20 kernels at 250 groups, the 80x80
-# kernels at 40 groups), mixed precision; traffic grows in proportion to the
+# kernels at 60 groups), mixed precision; traffic grows in proportion to the
 # cells, so a full launch is this times its cells.
 NCU_DRAM_BYTES_PER_CELL = {
     "water230_20": {
@@ -244,7 +244,7 @@ NCU_DRAM_BYTES_PER_CELL = {
         "source_energy": (249.24e6 + 132.63e6) / 44.1e6,
     },
     "water230_80": {
-        "transport": (420.0e6 + 366.8e6) / 104.976e6,  # transport_stream_kernel, 81x81x400x40
+        "transport": (630.1e6 + 576.4e6) / 157.464e6,  # transport_march_kernel, 81x81x400x60
     },
 }
 NCU_DRAM_BYTES_PER_CELL["bone230_80"] = NCU_DRAM_BYTES_PER_CELL["water230_80"]
