@@ -634,7 +634,7 @@ cudaError_t enq_lite_step(bfpn_ctx* c) {
     a.Ny = c->Ny;
     a.Nz = c->Nz;
     a.trapezoidal = (c->p.flags & BFPN_FLAG_TRAPEZOIDAL_YZ) ? 1 : 0;
-    const int n = energy_grid(c->elem, c->per_e, c->NA, true, true);  // consecutive lanes
+    const int n = lite_energy_grid(c->elem, c->per_e, c->NA);
     cudaError_t e = prof(c, BFPN_KERNEL_ENERGY, [&] { return launch_lite_energy<T>(a, c->stream); });
     if (e != cudaSuccess) return e;
     const double w = c->d.du * c->d.dv * c->d.dy * c->d.dz;

@@ -190,7 +190,7 @@ cudaError_t launch_finalize_idd_slots(const IddFinalArgs* args, int nslots, cuda
 template <typename T> cudaError_t launch_energy(const EnergyArgs<T>& a, cudaStream_t s);
 // Lite-memory primary step over psi^1 (F; f and src unused) with fused IDD
 // partials (psi^2 column 0); coef = [Ng][2] of tables.cpp: lite_coefficients;
-// energy_grid(elem, lanes, NA, true, true) partial pairs.
+// lite_energy_grid partial pairs.
 template <typename T> cudaError_t launch_lite_energy(const EnergyArgs<T>& a, cudaStream_t s);
 template <typename T> cudaError_t launch_transport(const TransportArgs<T>& a, int ang_chunk, cudaStream_t s);
 template <typename T> cudaError_t launch_angle(const AngleArgs<T>& a, cudaStream_t s);
@@ -323,6 +323,7 @@ size_t transport_plane_smem(int NP, int ac, size_t elem);
 // the most of any pass.
 int energy_grid(size_t elem, long long lanes, int NA, bool src, bool dose, int lanes_per_thread = 0);
 int energy_grid_most(size_t elem, long long lanes, int NA);
+int lite_energy_grid(size_t elem, long long lanes, int NA);
 // The passes whose lanes run in operand tiles: the primary's closing passes,
 // whose IDD partials the fused pass's are.
 __host__ __device__ constexpr bool energy_tiled(bool src, bool dose) { return dose && !src; }

@@ -75,7 +75,8 @@ __device__ __forceinline__ void store_lanes(double* p, const double (&x)[2]) {
 // Ring depth (groups) and groups per trip.  One lane per thread: 16 groups
 // deep, 4 per trip -- the few lanes of a small plane must cover the latency
 // alone.  Vectors: 6 deep, 2 per trip -- more blocks fit beside the constants.
-template <int LPT> struct RingShape { static constexpr int D = LPT == 1 ? 16 : 6, U = LPT == 1 ? 4 : 2; };
+constexpr int ring_depth(int lpt) { return lpt == 1 ? 16 : 6; }
+template <int LPT> struct RingShape { static constexpr int D = ring_depth(LPT), U = LPT == 1 ? 4 : 2; };
 
 // Constants of a group kept in shared memory (double2 each: psi^1 row, psi^2 row).
 template <int MODE, bool SRC>
@@ -381,8 +382,10 @@ __device__ __forceinline__ void energy_body(const EnergyArgs<T>& a, long long bi
     if (dose) block_partials(acc, accp, a.partials + 2 * bid);
 }
 
-// One register budget per form: the vector forms run two blocks of up to 160
-// threads beside each other, the scalar ones up to 640 threads alone.
+// One register budget per form: the vector forms run at least two blocks of up to
+// 160 threads (320 double) beside each other, all but the fused pass with
+// straggling, whose 220 registers leave one; the scalar ones one block of up to
+// 640 threads, or what its ring leaves of that (block_threads).
 template <int MODE, bool SRC, bool CS, typename T, int LPT>
 __global__ void __launch_bounds__(kEnergyMaxLanes / LPT) energy_kernel(EnergyArgs<T> a) {
     energy_body<MODE, SRC, CS, T, LPT>(a, blockIdx.x);
@@ -638,19 +641,28 @@ long long pass_threads(size_t elem, long long lanes, int NA, int lpt, bool tile)
     return 32 * ((lanes / NA + tp - 1) / tp) * ((NA + ta * lpt - 1) / (ta * lpt));
 }
 
-// Blocks of at most kEnergyMaxLanes lanes, as many for each SM (rounds), so the
-// last round is as full as the others; at least 128 lanes, so a block's warps
-// cover a copy's latency.
-int block_threads(long long threads, int lpt) {
-    const long long most = kEnergyMaxLanes / lpt, rounds = std::max<long long>(1, (threads + kEnergySMs * most - 1) / (kEnergySMs * most));
+// Shared memory a block's ring may take: what a block may have less the partial
+// sums' static array.
+constexpr size_t kEnergyRingLimit = 227 * 1024 - 512;
+
+// Blocks of at most kEnergyMaxLanes lanes and no more than have their ring of
+// `arrays` values in shared memory (576 threads for FP64 single lanes with a
+// source, at 384 bytes each; every other form's 640 lanes fit), as many for each
+// SM (rounds), so the last round is as full as the others; at least 128 lanes, so
+// a block's warps cover a copy's latency.
+int block_threads(long long threads, size_t elem, int lpt, int arrays) {
+    const size_t per_thread = static_cast<size_t>(ring_depth(lpt)) * arrays * lpt * elem;
+    const long long most = std::min<long long>(kEnergyMaxLanes / lpt, kEnergyRingLimit / per_thread / 32 * 32),
+                    rounds = std::max<long long>(1, (threads + kEnergySMs * most - 1) / (kEnergySMs * most));
     const long long per = (threads + kEnergySMs * rounds - 1) / (kEnergySMs * rounds);
     return static_cast<int>(std::max<long long>(128 / lpt, std::min<long long>(most, (per + 31) / 32 * 32)));
 }
 
+// arrays: what the pass's ring holds for a lane (psi^1, psi^2, the source).
 struct PassShape { int lpt, threads; unsigned grid; };
-PassShape pass_shape(size_t elem, long long lanes, int NA, int lpt, bool tile) {
+PassShape pass_shape(size_t elem, long long lanes, int NA, int lpt, int arrays, bool tile) {
     const long long n = pass_threads(elem, lanes, NA, lpt, tile);
-    const int b = block_threads(n, lpt);
+    const int b = block_threads(n, elem, lpt, arrays);
     return {lpt, b, static_cast<unsigned>((n + b - 1) / b)};
 }
 
@@ -671,7 +683,7 @@ cudaError_t launch_staged(int Ng, bool dose, int threads, const FS& in_smem, con
 
 template <int MODE, bool SRC, typename T, int LPT>
 cudaError_t launch_one(const EnergyArgs<T>& a, cudaStream_t s) {
-    const PassShape sh = pass_shape(sizeof(T), a.lanes, a.NA, LPT, energy_tiled(SRC, a.partials != nullptr));
+    const PassShape sh = pass_shape(sizeof(T), a.lanes, a.NA, LPT, SRC ? 3 : 2, energy_tiled(SRC, a.partials != nullptr));
     auto go = [&](auto kern, size_t smem) {
         cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
         if (e != cudaSuccess) return e;
@@ -686,7 +698,7 @@ cudaError_t launch_one(const EnergyArgs<T>& a, cudaStream_t s) {
 template <int MODE, bool SRC, int LPT>
 cudaError_t launch_slots(const EnergyArgs<float>* args, const int* begin, int nslots, int blocks, int max_ng,
                          long long lanes, int NA, bool dose, cudaStream_t s) {
-    const int threads = pass_shape(4, lanes, NA, LPT, energy_tiled(SRC, dose)).threads;
+    const int threads = pass_shape(4, lanes, NA, LPT, SRC ? 3 : 2, energy_tiled(SRC, dose)).threads;
     auto go = [&](auto kern, size_t smem) {
         cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
         if (e != cudaSuccess) return e;
@@ -700,7 +712,7 @@ cudaError_t launch_slots(const EnergyArgs<float>* args, const int* begin, int ns
 
 template <int MODE, int LPT>
 cudaError_t launch_fused(const EnergyFusedArgs& A, cudaStream_t s) {
-    const PassShape sh = pass_shape(4, A.e.lanes, A.e.NA, LPT, true);
+    const PassShape sh = pass_shape(4, A.e.lanes, A.e.NA, LPT, 2, true);
     auto go = [&](auto kern, size_t smem) {
         cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
         if (e != cudaSuccess) return e;
@@ -714,7 +726,7 @@ cudaError_t launch_fused(const EnergyFusedArgs& A, cudaStream_t s) {
 
 template <typename T, int LPT>
 cudaError_t launch_lite(const EnergyArgs<T>& a, cudaStream_t s) {
-    const PassShape sh = pass_shape(sizeof(T), a.lanes, a.NA, LPT, false);
+    const PassShape sh = pass_shape(sizeof(T), a.lanes, a.NA, LPT, 1, false);
     const size_t ring = ring_bytes<LPT, T>(sh.threads, 1), tab = energy_table_bytes(a.Ng, 1, true, true);
     const bool cs = tab + ring <= kEnergySmemLimit;
     auto kern = cs ? lite_energy_kernel<T, LPT, true> : lite_energy_kernel<T, LPT, false>;
@@ -729,11 +741,15 @@ cudaError_t launch_lite(const EnergyArgs<T>& a, cudaStream_t s) {
 
 int energy_grid(size_t elem, long long lanes, int NA, bool src, bool dose, int lanes_per_thread) {
     const int lpt = lanes_per_thread ? lanes_per_thread : vector_lanes(elem, lanes, NA);
-    return static_cast<int>(pass_shape(elem, lanes, NA, lpt, energy_tiled(src, dose)).grid);
+    return static_cast<int>(pass_shape(elem, lanes, NA, lpt, src ? 3 : 2, energy_tiled(src, dose)).grid);
+}
+
+int lite_energy_grid(size_t elem, long long lanes, int NA) {
+    return static_cast<int>(pass_shape(elem, lanes, NA, vector_lanes(elem, lanes, NA), 1, false).grid);
 }
 
 int energy_grid_most(size_t elem, long long lanes, int NA) {
-    int most = 0;
+    int most = lite_energy_grid(elem, lanes, NA);
     for (int lpt : {1, elem == 4 ? 4 : 2})
         for (bool src : {false, true}) most = std::max(most, energy_grid(elem, lanes, NA, src, true, lpt));
     return most;

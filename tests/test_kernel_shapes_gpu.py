@@ -14,6 +14,7 @@ import pytest
 from conftest import rel_err
 from test_parity_gpu import OP_TOL, STEP_TOL, assert_states, build, seeded_states, set_both, small_cfg
 from test_bundle_gpu import alone, check, pick
+from test_out_of_core_gpu import cfg_of, compare
 from bfpn_gpu_b200 import capi
 
 pytestmark = pytest.mark.gpu
@@ -49,6 +50,70 @@ def test_energy_sweep_shapes(shape, flags, precision):
     ctx.energy(0, 0.5 * cfg.dt())
     ora.energy(0, 0.5 * cfg.dt())
     assert_states(ctx, ora, OP_TOL if precision == capi.PREC_FP64 else 1e-6, ((0, 0), (0, 1)))
+
+
+# with a source (from 12 groups on these tables have one): 0 to 3 mod 4 groups;
+# the last three take one lane per thread in FP64 and balance to blocks of 608,
+# 640 and, over several rounds, 640 threads where the ring lets them
+SOURCED_SHAPES = [(6, 5, 4, 5, 40), (2, 8, 9, 1, 43), (3, 2, 3, 3, 17), (4, 4, 5, 7, 18), (17, 17, 16, 16, 16),
+                  (20, 21, 14, 14, 19), (26, 26, 11, 11, 16), (19, 19, 15, 15, 16), (100, 100, 9, 11, 12)]
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("flags", [{}, {"eq15_straggling": True, "trapezoidal_yz": True}, {"legacy_energy": True}])
+@pytest.mark.parametrize("shape", SOURCED_SHAPES)
+def test_sourced_energy_sweep_shapes(shape, flags, precision):
+    cfg = _energy_cfg(shape, **flags)
+    ctx, ora = build(cfg, precision=precision)
+    states = _states(ctx, 47, precision)
+    set_both(ctx, ora, states)
+    h = 0.5 * cfg.dt()
+    ora.energy(1, h)
+    plain = [ora.get_state(1, cf) for cf in (0, 1)]
+    ora.set_state(1, 0, states[2])
+    ora.set_state(1, 1, states[3])
+    ctx.secondary_source()
+    ora.source()
+    ctx.energy(1, h, with_source=True)
+    ora.energy(1, h, with_source=True)
+    if precision == capi.PREC_FP64:
+        assert_states(ctx, ora, OP_TOL, ((1, 0), (1, 1)))
+    added = 0.0
+    for cf in (0, 1):
+        want = ora.get_state(1, cf)
+        d = np.abs(want - plain[cf]).max()
+        # the sweep's own rounding, and the bar of the float source on what it adds
+        assert np.abs(ctx.get_state(1, cf) - want).max() <= 1e-6 * np.abs(want).max() + 2e-5 * d
+        added = max(added, d)
+    assert added > 0
+
+
+# a whole step at the same blocks: its IDD, summed from the sweeps' partials, is
+# that of the state it leaves.  Sums of double terms some 200 additions deep
+# (24 groups, a block's tree, its 150 blocks) in two orders: 1e-12 of the sum of
+# their magnitudes
+@pytest.mark.parametrize("ny,ang", [(26, 11), (19, 15)])
+def test_odd_angle_step_dose(ny, ang):
+    cfg = small_cfg(ny=ny, nz=ny, nmu=ang, nom=ang, ng=24)
+    ctx, _ = build(cfg)
+    ctx.step(1)  # the first step has no secondary half
+    for k, a in enumerate(_states(ctx, 48, capi.PREC_FP64)):
+        ctx.set_state(k // 2, k % 2, a)
+    got = ctx.step(1)[0][0]
+    want = ctx.idd()[0]
+    left = [ctx.get_state(k // 2, k % 2) for k in range(4)]
+    terms = 0.0
+    for keep in (0, 1):
+        for k, a in enumerate(left):
+            ctx.set_state(k // 2, k % 2, np.abs(a) if k % 2 == keep else np.zeros_like(a))
+        terms += abs(ctx.idd()[0])
+    assert np.abs(left[2]).max() > 0 and terms > 0
+    assert abs(got - want) <= 1e-12 * terms
+
+
+def test_out_of_core_odd_angle_chunks():
+    """Lane chunks of 33 x 33 positions x 81 angles (608 threads), the last partial."""
+    compare(cfg_of(ny=49, nz=49, nmu=9, nom=9, ng=24, ly=8.0, lz=8.0, t_final=0.5), capi.PREC_FP64, 4, (1089 * 81, 5))
 
 
 @pytest.mark.parametrize("straggling", [False, True])
