@@ -310,3 +310,31 @@ def test_bundle_tuning_lengths(n):
         assert b.running() == 0
         for s, ref in zip(slots, refs):
             check(b.collect(s), ref)
+
+
+def _page_locked_kb():
+    """Page-locked host memory that the driver has mapped into this process."""
+    kb = 0
+    with open("/proc/self/maps") as maps:
+        for line in maps:
+            if "/dev/zero" in line:
+                lo, hi = line.split()[0].split("-")
+                kb += (int(hi, 16) - int(lo, 16)) // 1024
+    return kb
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+def test_step_calls_lock_no_memory(precision):
+    """The buffer of a step call's results is no allocation of page-locked memory
+    (which takes longer than the step of a small beam); the first calls, which
+    copy, and the later ones give the history."""
+    cfg = small_cfg()
+    ctx, _ = build(cfg, precision=precision)
+    ctx.step_async(2)
+    ctx.sync()
+    before = _page_locked_kb()
+    got = [ctx.step(n) for n in [1] * 15 + [3, 2, 1, 256]]
+    assert _page_locked_kb() == before
+    idd, prox = ctx.history()
+    assert np.array_equal(np.concatenate([g[0] for g in got]), idd[2:])
+    assert np.array_equal(np.concatenate([g[1] for g in got]), prox[2:])
