@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -218,6 +219,24 @@ void drop_graphs(bfpn_ctx* c) {
     }
 }
 
+constexpr size_t kPage = 4096;
+
+// Page-locks whole pages of host memory in place, allowed while another thread
+// captures a graph; false (no error left behind) where that cannot be had.
+bool lock_pages(void* p, size_t bytes) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaHostRegister(p, bytes, cudaHostRegisterMapped);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
+}
+void free_pages(void*& p, bool locked) {
+    if (p && locked) cudaHostUnregister(p);
+    std::free(p);
+    p = nullptr;
+}
+
 void free_all(bfpn_ctx* c) {
     for (auto& p : c->pending) {
         cudaEventDestroy(p.a);
@@ -241,11 +260,7 @@ void free_all(bfpn_ctx* c) {
     c->allocs.clear();
     for (void* p : c->host_allocs) cudaFreeHost(p);
     c->host_allocs.clear();
-    if (c->step_export) {
-        cudaHostUnregister(c->step_export);
-        std::free(c->step_export);
-        c->step_export = nullptr;
-    }
+    free_pages(c->step_export, true);
 }
 
 // Transport launch shape: a whole (Ny+1) x (Nz+1) plane per block when it
@@ -1346,52 +1361,50 @@ bfpn_status check_device_error(bfpn_ctx* c) {
     return fail(c, BFPN_TIMEOUT, "a bounded device wait ran out (code " + std::to_string(h) + "); results of the step are invalid");
 }
 
-// The results of one bfpn_step call -- up to kExportSteps IDD and proxy values
-// and the device error word -- written by one small kernel into pinned memory
-// the host reads after a single wait: 0.010 ms, against 0.039 ms for three pageable
-// copies, each with its own wait.  The buffer is two pages of ordinary memory
-// registered with the device, which costs 0.28 ms and 0.17 ms to give back (a
-// pinned allocation took 0.9 to 2.6 ms in each context's first call); so a context
-// registers it after as many calls as would have repaid it, and a program that
-// makes few calls pays for none.
-constexpr int kExportAfter = 16;
-constexpr int kExportSteps = 256;
+// The results of one bfpn_step call -- up to kExportSteps IDD and proxy values and
+// the device error word -- packed by one small kernel and read after a single wait
+// (three pageable copies, each with its own wait, take 0.039 ms, as long as several
+// kernels of a small beam's step).  The kernel writes to device memory, from where
+// one pageable copy brings them (0.016 ms in all), or, once a context has made
+// kExportAfter such calls, into host memory registered with the device (0.010 ms).
+// That memory is two ordinary pages, 0.28 ms to register and 0.17 ms to give back, so
+// a program that makes few calls should not pay for it; a pinned allocation took 0.9
+// to 2.6 ms in each context's first call.
+constexpr int kExportSteps = 256, kExportAfter = 32;
 struct StepExport {
-    double idd[kExportSteps], proxy[kExportSteps];
-    int err;
+    int err, unused;
+    double v[2 * kExportSteps];  // count IDD values, count proxy values
 };
 
-// The buffer, registered on first use and allowed while another thread captures a
-// graph; false (no error left behind) where there is none to be had.
-bool export_ready(bfpn_ctx* c) {
-    if (c->step_export) return true;
-    constexpr size_t page = 4096, bytes = (sizeof(StepExport) + page - 1) / page * page;
-    void* p = std::aligned_alloc(page, bytes);
-    if (!p) return false;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    const cudaError_t e = cudaHostRegister(p, bytes, cudaHostRegisterMapped);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
+// The registered pages; null before they are due and where there are none to be had.
+StepExport* export_pages(bfpn_ctx* c) {
+    if (c->step_export || ++c->step_calls <= kExportAfter) return static_cast<StepExport*>(c->step_export);
+    c->step_calls = 0;  // (asked for again after as many calls if it fails)
+    constexpr size_t bytes = (sizeof(StepExport) + kPage - 1) / kPage * kPage;
+    void* p = std::aligned_alloc(kPage, bytes);
+    if (!p || !lock_pages(p, bytes)) {
         std::free(p);
-        return false;
+        return nullptr;
     }
     c->step_export = p;
-    return true;
+    return static_cast<StepExport*>(p);
 }
 
-// (the buffer is there)
 bfpn_status export_history(bfpn_ctx* c, int first, int count, double* idd_out, double* proxy_out, bool* clean) {
-    auto* h = static_cast<StepExport*>(c->step_export);
-    void* d = nullptr;
-    CUDA_TRY(c, cudaHostGetDevicePointer(&d, h, 0));
+    StepExport copy, *h = export_pages(c);
+    void* d = c->step_result;
+    if (h) CUDA_TRY(c, cudaHostGetDevicePointer(&d, h, 0));
     auto* dv = static_cast<StepExport*>(d);
-    CUDA_TRY(c, launch_export_history(c->hist_idd + first, c->hist_proxy + first, count, c->dev_err, dv->idd, dv->proxy,
+    CUDA_TRY(c, launch_export_history(c->hist_idd + first, c->hist_proxy + first, count, c->dev_err, dv->v, dv->v + count,
                                       &dv->err, c->stream));
+    if (!h) {
+        h = &copy;
+        CUDA_TRY(c, cudaMemcpyAsync(h, dv, offsetof(StepExport, v) + 2 * count * sizeof(double), cudaMemcpyDeviceToHost,
+                                    c->stream));
+    }
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    if (idd_out) std::memcpy(idd_out, h->idd, count * sizeof(double));
-    if (proxy_out) std::memcpy(proxy_out, h->proxy, count * sizeof(double));
+    if (idd_out) std::memcpy(idd_out, h->v, count * sizeof(double));
+    if (proxy_out) std::memcpy(proxy_out, h->v + count, count * sizeof(double));
     *clean = h->err == 0;
     return BFPN_OK;
 }
@@ -1651,6 +1664,7 @@ bfpn_status bfpn_create(const bfpn_grid* grid, const bfpn_phys* phys, int precis
     ALLOC(c->counter, sizeof(int));
     ALLOC(c->zero_counter, sizeof(int));
     ALLOC(c->dev_err, sizeof(int));
+    ALLOC(c->step_result, sizeof(StepExport));
     ALLOC(c->scalar_out, 2 * sizeof(double));
     ALLOC(c->moments, 2 * static_cast<size_t>(c->Ng) * sizeof(double));
     ALLOC(c->plane, static_cast<size_t>(c->nyz) * sizeof(double));
@@ -1948,7 +1962,7 @@ bfpn_status bfpn_step(bfpn_ctx* c, int32_t nsteps, double* idd_out, double* prox
     const int first = c->steps_done;
     bfpn_status s = bfpn_step_async(c, nsteps);
     if (s != BFPN_OK) return s;
-    if (nsteps > 0 && nsteps <= kExportSteps && (c->step_export || ++c->step_calls > kExportAfter) && export_ready(c)) {
+    if (nsteps > 0 && nsteps <= kExportSteps) {
         bool clean = false;
         if ((s = export_history(c, first, nsteps, idd_out, proxy_out, &clean)) != BFPN_OK) return s;
         CUDA_TRY(c, collect_profile(c));

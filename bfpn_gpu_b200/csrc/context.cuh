@@ -65,8 +65,9 @@ struct bfpn_ctx {
     int hist_cap = 0;
     int* counter = nullptr;
     void* stage[2] = {};            // pinned buffers of large state transfers (in host_allocs)
-    void* step_export = nullptr;    // registered, mapped: results of one step call
-    int step_calls = 0;             // bfpn_step calls before that
+    void* step_result = nullptr;    // device: the results of one step call
+    void* step_export = nullptr;    // registered host pages in its place
+    int step_calls = 0;             // step calls before those
     int* zero_counter = nullptr;    // scratch counter for one-off IDD reductions
     int* dev_err = nullptr;         // device error word (bounded waits that ran out)
     void* bblob = nullptr;          // split-bf16 angular kernel tiles for the tensor-core source

@@ -327,13 +327,13 @@ def _page_locked_kb():
 def test_step_calls_lock_no_memory(precision):
     """The buffer of a step call's results is no allocation of page-locked memory
     (which takes longer than the step of a small beam); the first calls, which
-    copy, and the later ones give the history."""
+    copy, and the later ones, which do not, give the history."""
     cfg = small_cfg()
     ctx, _ = build(cfg, precision=precision)
     ctx.step_async(2)
     ctx.sync()
     before = _page_locked_kb()
-    got = [ctx.step(n) for n in [1] * 15 + [3, 2, 1, 256]]
+    got = [ctx.step(n) for n in [1, 256] + [1] * 29 + [3, 2, 1, 256]]
     assert _page_locked_kb() == before
     idd, prox = ctx.history()
     assert np.array_equal(np.concatenate([g[0] for g in got]), idd[2:])
