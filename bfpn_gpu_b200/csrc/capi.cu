@@ -261,6 +261,7 @@ void free_all(bfpn_ctx* c) {
     for (void* p : c->host_allocs) cudaFreeHost(p);
     c->host_allocs.clear();
     free_pages(c->step_export, true);
+    for (int k = 0; k < 2; ++k) free_pages(c->stage[k], c->stage_locked[k]);
 }
 
 // Transport launch shape: a whole (Ny+1) x (Nz+1) plane per block when it
@@ -351,11 +352,17 @@ bool transport_in_place(const bfpn_ctx* c) {
 }
 
 // A large array between the caller's doubles and device values of T: chunks go
-// through two pinned buffers of the context (2 MB each, allocated on first use)
-// while host threads convert the neighbouring chunk, so the link, the conversion
-// and the page faults of a fresh caller buffer overlap.  (A pageable copy into a
-// zeroed temporary and a serial conversion took 10 ms for 3.4M floats.)
-constexpr size_t kStageBytes = size_t(2) << 20, kStageSmall = size_t(8) << 20;  // smaller arrays do not repay the buffers
+// through two host buffers of the context (2 MB each, allocated on first use) while
+// host threads convert the neighbouring chunk, so the link, the conversion and the
+// page faults of a fresh caller buffer overlap.  (One pageable copy into a zeroed
+// temporary and a serial conversion took 10 ms for 3.4M floats.)  The buffers are
+// ordinary memory at first, through which the driver's own staging moves 13 GB/s down
+// and 20 GB/s up, and are page-locked in place for the transfer with which a context
+// has moved kStageLock bytes: that takes 1 to 4 ms (allocating them locked took 2 to
+// 12 ms, more than the first transfer of up to 20M values) and saves 0.045 ms for each
+// MB.
+constexpr size_t kStageBytes = size_t(2) << 20, kStageLock = size_t(128) << 20;
+constexpr size_t kStageSmall = size_t(8) << 20;  // smaller arrays do not repay the threads
 
 template <typename T>
 void convert_values(T* dev_side, double* host, size_t n, bool up) {
@@ -366,27 +373,17 @@ void convert_values(T* dev_side, double* host, size_t n, bool up) {
     }
 }
 
-// Pinned memory of the context, allocated on first use and allowed while another
-// thread captures a graph; false (no error left behind) where there is none to be
-// had: the caller then takes its path through pageable memory.
-bool host_buffer(bfpn_ctx* c, void*& p, size_t bytes, unsigned flags) {
-    if (p) return true;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    const cudaError_t e = cudaHostAlloc(&p, bytes, flags);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        p = nullptr;
-        return false;
+// The buffers for a transfer of `bytes` of device values; false where there are none.
+bool stage_ready(bfpn_ctx* c, size_t bytes) {
+    for (void*& p : c->stage)
+        if (!p && !(p = std::aligned_alloc(kPage, kStageBytes))) return false;
+    c->staged += bytes;
+    if (c->staged >= kStageLock && !(c->stage_locked[0] && c->stage_locked[1])) {
+        for (int k = 0; k < 2; ++k)
+            c->stage_locked[k] = c->stage_locked[k] || lock_pages(c->stage[k], kStageBytes);
+        c->staged = 0;  // (if it failed: tried again as far on)
     }
-    c->host_allocs.push_back(p);
     return true;
-}
-
-bool stage_ready(bfpn_ctx* c) {
-    return host_buffer(c, c->stage[0], kStageBytes, cudaHostAllocDefault) &&
-           host_buffer(c, c->stage[1], kStageBytes, cudaHostAllocDefault);
 }
 
 // (stage_ready came first)
@@ -454,7 +451,7 @@ bfpn_status staged_transfer(bfpn_ctx* c, void* dev, double* host, size_t n, bool
 
 template <typename T>
 bfpn_status upload_as(bfpn_ctx* c, void* dst, const double* host, size_t n) {
-    if (n * sizeof(T) > kStageSmall && stage_ready(c))
+    if (n * sizeof(T) > kStageSmall && stage_ready(c, n * sizeof(T)))
         return staged_transfer<T>(c, dst, const_cast<double*>(host), n, true);
     if (sizeof(T) == sizeof(double)) {
         CUDA_TRY(c, cudaMemcpyAsync(dst, host, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
@@ -1334,7 +1331,7 @@ bfpn_status run_steps(bfpn_ctx* c, int nsteps) {
 
 template <typename T>
 bfpn_status download_as(bfpn_ctx* c, const void* dev, double* host, size_t n) {
-    if (n * sizeof(T) > kStageSmall && stage_ready(c))
+    if (n * sizeof(T) > kStageSmall && stage_ready(c, n * sizeof(T)))
         return staged_transfer<T>(c, const_cast<void*>(dev), host, n, false);
     if (sizeof(T) == sizeof(double)) {
         CUDA_TRY(c, cudaMemcpyAsync(host, dev, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));

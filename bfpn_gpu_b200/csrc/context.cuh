@@ -64,7 +64,9 @@ struct bfpn_ctx {
     double* hist_proxy = nullptr;
     int hist_cap = 0;
     int* counter = nullptr;
-    void* stage[2] = {};            // pinned buffers of large state transfers (in host_allocs)
+    void* stage[2] = {};            // host buffers of large state transfers (whole pages)
+    bool stage_locked[2] = {};      // page-locked, once `staged` bytes went through them
+    size_t staged = 0;
     void* step_result = nullptr;    // device: the results of one step call
     void* step_export = nullptr;    // registered host pages in its place
     int step_calls = 0;             // step calls before those

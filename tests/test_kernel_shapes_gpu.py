@@ -338,3 +338,18 @@ def test_step_calls_lock_no_memory(precision):
     idd, prox = ctx.history()
     assert np.array_equal(np.concatenate([g[0] for g in got]), idd[2:])
     assert np.array_equal(np.concatenate([g[1] for g in got]), prox[2:])
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+def test_large_transfers_lock_no_memory(precision):
+    """A context's first large state transfers allocate no page-locked memory
+    (which takes longer than the transfer), and later ones through buffers locked
+    in place (from 128 MB on) bring the same values."""
+    cfg = small_cfg(ny=16, nz=16, nmu=16, nom=16, ng=40)
+    ctx, _ = build(cfg, precision=precision)
+    before = _page_locked_kb()
+    a = (np.arange(int(np.prod(ctx.shape))) % 4093).astype(np.float64)
+    for k in range(8):
+        ctx.set_state(k // 2 % 2, k % 2, a + k)
+        assert np.array_equal(ctx.get_state(k // 2 % 2, k % 2), a + k)
+    assert _page_locked_kb() == before
