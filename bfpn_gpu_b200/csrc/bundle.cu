@@ -38,8 +38,11 @@ using namespace bfpn;
 namespace {
 
 constexpr int kMaxSideStreams = 4;
-constexpr int kTuneSteps = 6;        // depth steps of one tuning run
+constexpr int kTunePairs = 3;        // pairs of depth steps of one tuning run, the first untimed
 constexpr int kBundleMaxPlane = 65;  // Ny + 1 and Nz + 1 of a bundle's beams
+
+// Kernel classes timed by the autotuner.
+enum { TK_ENERGY = 0, TK_TRANSPORT = 1, TK_ANGLE = 2, TK_N = 3 };
 
 struct Tuning {
     bool tuned = false;
@@ -93,6 +96,8 @@ struct bfpn_bundle {
     long long lanes = 0;
     bool no_clip = false;
     Tuning tune;
+    int tune_pairs = 0;           // tuning pairs taken
+    double tune_ms[2][TK_N] = {};  // least times of sets A and B
     bool autotune = true;
     // device argument image and the graph of the current slot set
     void* dimg = nullptr;
@@ -264,9 +269,6 @@ cudaError_t enq_angle_t(bfpn_bundle* b, const LaunchTable& t, cudaStream_t s) {
                               b->tune.dst_stages, s);
 }
 
-// Kernel classes timed by the autotuner.
-enum { TK_ENERGY = 0, TK_TRANSPORT = 1, TK_ANGLE = 2, TK_N = 3 };
-
 // One depth step of the planned slots on b->stream.  times != null: eager,
 // each timed class bracketed by events and its milliseconds added.
 cudaError_t enq_bundle_step(bfpn_bundle* b, double* times) {
@@ -350,53 +352,57 @@ bfpn_status ensure_plan(bfpn_bundle* b, const std::vector<int>& prim, const std:
     return BFPN_OK;
 }
 
-// Autotuning: three eager steps per variant set, A and B alternating (A B A B
-// A B), each kernel class keeps its faster variant by the last pair: the steps
-// before load the code of its kernels (the secondary's from the second step on),
-// which takes up to 30 ms and would decide the choice.  Beams too short for
-// that run set A untuned.  The steps are real steps of the bundle.  Returns the
-// steps taken.
-bfpn_status autotune(bfpn_bundle* b, const std::vector<int>& prim, int max_steps, int* taken) {
-    *taken = 0;
-    Tuning A = b->tune, B = b->tune;
+// Autotuning: pairs of eager steps, the first of a pair with variant set A, the
+// second with B; each kernel class keeps its faster variant by the least time of
+// the pairs after the first, which loads the code of the kernels (up to 30 ms, which
+// would decide the choice).  The steps are real steps of the bundle, in which every
+// slot runs both halves, so that both sets do the same work; between pairs, and
+// until the last one is taken, the bundle runs set A.  The pairs may come in
+// different calls and from different beams: what a bundle learned is kept while
+// short calls or short beams leave room for a pair only now and then.
+bfpn_status tuning_pair(bfpn_bundle* b, const std::vector<int>& prim) {
+    const Tuning was = b->tune;
+    Tuning A = was, B = was;
     A.tr_ac = 16;
     B.tr_ac = 8;
     A.dst_stages = 2;
     B.dst_stages = 3;
     A.ring = true;
     B.ring = false;
-    double warm[TK_N] = {}, tA[TK_N] = {}, tB[TK_N] = {};
-    const int rounds = std::min(kTuneSteps, max_steps);
-    for (int r = 0; r < rounds; ++r) {
-        b->tune = (r % 2 == 0) ? A : B;
-        // a slot's first step has no secondary half
-        std::vector<int> sec_now;
-        for (int s : prim)
-            if (b->slots[s].ctx->steps_done > 0) sec_now.push_back(s);
-        bfpn_status st = ensure_plan(b, prim, sec_now, false);
+    for (int v = 0; v < 2; ++v) {
+        double ms[TK_N] = {};
+        b->tune = v == 0 ? A : B;
+        bfpn_status st = ensure_plan(b, prim, prim, false);
+        const cudaError_t e = st == BFPN_OK ? enq_bundle_step(b, ms) : cudaSuccess;
+        b->plan_sig.clear();
+        b->tune = A;
         if (st != BFPN_OK) return st;
-        cudaError_t e = enq_bundle_step(b, r < 4 ? warm : (r % 2 == 0) ? tA : tB);
         if (e != cudaSuccess) return bfail(b, BFPN_CUDA_ERROR, std::string("bundle tuning step: ") + cudaGetErrorString(e));
         for (int s : prim) b->slots[s].ctx->steps_done += 1;
-        ++*taken;
-        b->plan_sig.clear();
+        for (int k = 0; k < TK_N; ++k) {
+            double& t = b->tune_ms[v][k];
+            if (b->tune_pairs == 1 || ms[k] < t) t = ms[k];  // (the first pair's time is dropped)
+        }
     }
+    if (++b->tune_pairs < kTunePairs) return BFPN_OK;
+    const auto& tA = b->tune_ms[0];
+    const auto& tB = b->tune_ms[1];
     Tuning best = A;
-    if (rounds == kTuneSteps) {
-        const bool fixed_tr = b->cl || b->march;  // one transport form: nothing to choose
-        best.tr_ac = (fixed_tr || tA[TK_TRANSPORT] <= tB[TK_TRANSPORT]) ? A.tr_ac : B.tr_ac;
-        best.dst_stages = tA[TK_ANGLE] <= tB[TK_ANGLE] ? A.dst_stages : B.dst_stages;
-        best.ring = tA[TK_ENERGY] <= tB[TK_ENERGY] ? A.ring : B.ring;
-        best.tuned = true;
-        char buf[320];
-        std::snprintf(buf, sizeof buf,
-                      "%s: transport %s (%.3f ms vs %.3f ms per step), DST %d stages (%.3f vs %.3f), "
-                      "energy %s (%.3f vs %.3f)",
-                      b->key.c_str(),
-                      b->march ? "marching" : b->cl ? "cluster" : (best.tr_ac == 16 ? "16 angles/block" : "8 angles/block"),
-                      tA[TK_TRANSPORT], tB[TK_TRANSPORT], best.dst_stages, tA[TK_ANGLE], tB[TK_ANGLE],
-                      best.ring ? "4 lanes per thread" : "1 lane per thread", tA[TK_ENERGY], tB[TK_ENERGY]);
-        best.report = buf;
+    const bool fixed_tr = b->cl || b->march;  // one transport form: nothing to choose
+    best.tr_ac = (fixed_tr || tA[TK_TRANSPORT] <= tB[TK_TRANSPORT]) ? A.tr_ac : B.tr_ac;
+    best.dst_stages = tA[TK_ANGLE] <= tB[TK_ANGLE] ? A.dst_stages : B.dst_stages;
+    best.ring = tA[TK_ENERGY] <= tB[TK_ENERGY] ? A.ring : B.ring;
+    best.tuned = true;
+    char buf[320];
+    std::snprintf(buf, sizeof buf,
+                  "%s: transport %s (%.3f ms vs %.3f ms per step), DST %d stages (%.3f vs %.3f), "
+                  "energy %s (%.3f vs %.3f)",
+                  b->key.c_str(),
+                  b->march ? "marching" : b->cl ? "cluster" : (best.tr_ac == 16 ? "16 angles/block" : "8 angles/block"),
+                  tA[TK_TRANSPORT], tB[TK_TRANSPORT], best.dst_stages, tA[TK_ANGLE], tB[TK_ANGLE],
+                  best.ring ? "4 lanes per thread" : "1 lane per thread", tA[TK_ENERGY], tB[TK_ENERGY]);
+    best.report = buf;
+    {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         g_tune[b->key] = best;
     }
@@ -574,11 +580,10 @@ bfpn_status bfpn_bundle_step(bfpn_bundle* b, int32_t nsteps) {
             min_rest = std::min(min_rest, s.nsteps - s.ctx->steps_done);
         }
         if (prim.empty()) break;
-        if (b->autotune && !b->tune.tuned && min_rest >= kTuneSteps) {
-            int taken = 0;
-            bfpn_status st = autotune(b, prim, min_rest, &taken);
+        if (b->autotune && !b->tune.tuned && min_rest >= 2 && sec.size() == prim.size()) {
+            bfpn_status st = tuning_pair(b, prim);
             if (st != BFPN_OK) return st;
-            left -= taken;
+            left -= 2;
             continue;
         }
         // a slot's first step has no secondary half: one step with that plan

@@ -424,9 +424,10 @@ bfpn_status bfpn_batch_run(const bfpn_beam* beams, int32_t n, const int32_t* dev
  * tables, beam, depth-step count and IDD history, and join or leave at any
  * step (continuous batching).  The step of the current slot set is one CUDA
  * graph.  Kernel variants (angles per transport block, DST ring stages,
- * lanes per energy thread) are timed per shape class on six of the bundle's
- * steps, the first four of which only load the kernels (beams with fewer steps
- * left run the defaults), and the fastest kept for the process (autotuning);
+ * lanes per energy thread) are timed per shape class on three pairs of the
+ * bundle's steps, the first of which only loads the kernels (a pair needs two
+ * steps left of every beam and of the call; until the third the bundle runs the
+ * defaults), and the fastest kept for the process (autotuning);
  * all variants compute the
  * same states.  Each beam's IDD history equals its single-context run up to
  * the order of the IDD partial sums. */

@@ -312,6 +312,23 @@ def test_bundle_tuning_lengths(n):
             check(b.collect(s), ref)
 
 
+# classes that no other test uses: the choice is kept for the process
+@pytest.mark.parametrize("ny,na,n,call", [(14, 8, 9, 2), (12, 16, 5, 1000)])
+def test_bundle_tunes_in_short_runs(ny, na, n, call):
+    """Calls of two steps, and beams of five one after another, tune the bundle as
+    longer ones do."""
+    reqs = pick(ny, na, 2, n)
+    with capi.Bundle(max_slots=1) as b:
+        assert b.tuning() == "not tuned"
+        for r in reqs:
+            ref = alone(r)
+            slot = b.admit(r.beam())
+            while b.running():
+                b.step(call)
+            check(b.collect(slot), ref)
+        assert "lane" in b.tuning()
+
+
 def _page_locked_kb():
     """Page-locked host memory that the driver has mapped into this process."""
     kb = 0
