@@ -2234,7 +2234,14 @@ bfpn_status bfpn_table_download(bfpn_ctx* c, int32_t which, double* host, uint64
     if (!c || !host) return BFPN_INVALID_ARG;
     if (!c->tables_loaded) return fail(c, BFPN_NOT_READY, "tables not loaded");
     std::vector<double> tmp;
-    if (which == BFPN_TABLE_KER_V) angular_kernel_f64(c->tables);
+    if (which == BFPN_TABLE_KER_V) {
+        const size_t size = static_cast<size_t>(c->Ng) * c->NA * c->NA;
+        if (c->prec == BFPN_PREC_FP64 && c->ker_v && size <= n) {  // the one in use
+            bfpn_status s = set_device(c);
+            return s != BFPN_OK ? s : download_as<double>(c, c->ker_v, host, size);
+        }
+        angular_kernel_f64(c->tables);
+    }
     const TableView src = table_of(c->tables, which, tmp);
     if (!src.known) return fail(c, BFPN_INVALID_ARG, "unknown table id");
     if (src.size > n) return fail(c, BFPN_INVALID_ARG, "host buffer too small for the table");

@@ -220,7 +220,12 @@ bfpn_status bfpn_state_download(bfpn_ctx* ctx, int32_t species, int32_t coef, do
 bfpn_status bfpn_source_download(bfpn_ctx* ctx, double* host);
 uint64_t bfpn_cells(const bfpn_ctx* ctx);
 
-/* One set-up table (BFPN_TABLE_*); n = capacity of host in doubles. */
+/* One set-up table (BFPN_TABLE_*); n = capacity of host in doubles.
+ * BFPN_TABLE_KER_V: a FP64 context returns the table it uses, which it built on
+ * the device.  A mixed-precision context uses the float rounding of that build and
+ * returns the host's double build (as bfpn_host_table), which differs from the
+ * device's in the last bits of acos, pow and exp; an entry within those bits of the
+ * threshold 1e-3 may be dropped in one and kept in the other. */
 bfpn_status bfpn_table_download(bfpn_ctx* ctx, int32_t which, double* host, uint64_t n);
 
 /* Kernel classes of the per-kernel profile. */

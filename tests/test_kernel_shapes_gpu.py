@@ -11,11 +11,11 @@ the angular step (4 * 32 * 2^-24 = 8e-6, bar 2e-5)."""
 import numpy as np
 import pytest
 
-from conftest import rel_err
+from conftest import rel_err, table_dir
 from test_parity_gpu import OP_TOL, STEP_TOL, assert_states, build, seeded_states, set_both, small_cfg
 from test_bundle_gpu import alone, check, pick
 from test_out_of_core_gpu import cfg_of, compare
-from bfpn_gpu_b200 import capi
+from bfpn_gpu_b200 import capi, read_tables
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -327,6 +327,34 @@ def test_bundle_tunes_in_short_runs(ny, na, n, call):
                 b.step(call)
             check(b.collect(slot), ref)
         assert "lane" in b.tuning()
+
+
+def test_downloaded_angular_kernel_is_the_one_in_use():
+    """Unit values of psi^1, one direction at each position: the source is the
+    group's angular kernel times its energy kernel and the group width, product by
+    product, so the table a FP64 context returns gives it bit for bit.  Against the
+    host's build of that table the entries agree to the last bits of acos, pow and
+    exp (a few 1e-16 each, times exponents below 100: 1e-12), but for one within
+    those of the threshold 1e-3, which either side may drop."""
+    cfg = small_cfg(ny=6, nz=6, nmu=6, nom=8)
+    ctx, _ = build(cfg)
+    Ng, nyz, NA = ctx.shape
+    K = ctx.table(capi.TABLE_KER_V, Ng * NA * NA).reshape(Ng, NA, NA)
+    e1 = ctx.table(capi.TABLE_KER_E1, Ng * Ng).reshape(Ng, Ng)
+    for s in (2, 7, 20):
+        F = np.zeros((Ng, nyz, NA))
+        F[s, np.arange(nyz), np.arange(nyz) % NA] = 1.0
+        ctx.set_state(0, 0, F.ravel())
+        ctx.set_state(0, 1, np.zeros(F.size))
+        ctx.secondary_source()
+        want = cfg.grid().Lg / Ng * (e1[:, s, None, None] * K[s][np.arange(nyz) % NA][None])
+        assert np.count_nonzero(want) > nyz
+        assert np.array_equal(ctx.source().reshape(Ng, nyz, NA), want)
+    mu, sig = read_tables(table_dir("synthetic500"), cfg.ng)
+    H = capi.host_table(cfg.grid(), cfg.phys(), mu, sig, capi.TABLE_KER_V).reshape(K.shape)
+    one = (K == 0) != (H == 0)
+    assert np.all(np.abs(np.maximum(K, H)[one] - 1e-3) <= 1e-15)
+    assert np.all(np.abs(K - H)[~one] <= 1e-12 * H[~one])
 
 
 def _page_locked_kb():
