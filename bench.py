@@ -233,18 +233,22 @@ def kernel_bytes(cls, cells, elem, n_groups, nyz, NA, fused=False):
 # DRAM bytes (read + write) per cell of one launch of each kernel class, from ncu
 # captures of the same kernels on a smaller state of the same lateral and
 # angular grid (profiles/*.txt: the 20x20 kernels at 250 groups, the 80x80
-# kernels at 60 groups), mixed precision; traffic grows in proportion to the
-# cells, so a full launch is this times its cells.
+# transport at 60 groups, its energy sweep with a source and DST at 30), mixed
+# precision; traffic grows in proportion to the cells, so a full launch is this
+# times its cells.  The fused pass and the source also move data by source group.
 NCU_DRAM_BYTES_PER_CELL = {
     "water230_20": {
-        "transport": (176.52e6 + 122.73e6) / 44.1e6,
-        "angle": (176.85e6 + 119.49e6) / 44.1e6,
-        "energy": (352.90e6 + 295.12e6) / 44.1e6,
-        "source_angular": (190.52e6 + 153.69e6 + 284.85e6 + 154.88e6) / 44.1e6,  # pack + GEMM
-        "source_energy": (249.24e6 + 132.63e6) / 44.1e6,
+        "transport": (176.5e6 + 122.7e6) / 44.1e6,
+        "angle": (176.9e6 + 118.6e6) / 44.1e6,
+        "energy": (531.2e6 + 301.1e6) / 44.1e6,
+        "energy_fused": (382.0e6 + 495.9e6) / 44.1e6,
+        "source_angular": (252.2e6 + 154.0e6) / 44.1e6,  # no pack: the fused pass writes its operand
+        "source_energy": (249.2e6 + 133.6e6) / 44.1e6,
     },
     "water230_80": {
         "transport": (630.1e6 + 576.4e6) / 157.464e6,  # transport_march_kernel, 81x81x400x60
+        "angle": (315.1e6 + 257.0e6) / 78.732e6,
+        "energy": (944.9e6 + 577.1e6) / 78.732e6,
     },
 }
 NCU_DRAM_BYTES_PER_CELL["bone230_80"] = NCU_DRAM_BYTES_PER_CELL["water230_80"]

@@ -118,7 +118,7 @@ struct bfpn_ctx {
     bool tr_pairs = true;       // use the paired kernel where it applies
     bool tr_cluster_ok = false; // a cluster kernel is compiled for this plane (float state)
     int tr_cluster = 1;         // 0 off, 1 planes without a whole-plane kernel, 2 every supported plane
-    bool tr_stream_ok = false;  // the row-streaming kernel applies (float state, plane <= 128 wide)
+    bool tr_stream_ok = false;  // the row-streaming kernel applies (float state, plane <= 256 wide; the march goes before it)
     int tr_stream = 1;          // 0 off, 1 planes without a whole-plane kernel, 2 every supported plane
     bool tr_tile_ok = false;    // the plane needs tiles: the unrolled tiled kernel applies
     bool tr_tile = false;       // use it

@@ -9,9 +9,10 @@
 // run-time-length kernel reads two operands per product: 15 x 12 angles took
 // 1.36 ms for 62M float cells, 0.29 here).  The transforms are compiled per length and
 // picked by a block-uniform switch; a kernel is compiled for lengths up to 8,
-// 16, 24 and 32, since the longest sets its registers.  What bounds it: the fma
-// pipe and, between the passes, the block's barriers, which the other blocks of
-// the SM cover.
+// 16, 24 and 32, since the longest sets its registers.  What bounds it: latency -- a
+// whole line per thread takes 148 registers at 15 x 12 angles, so 18 % of the
+// warps are there to cover a line's chains and the block's barriers (issue 44 %, fma
+// pipe 41 % busy).
 #include "common.cuh"
 #include "dst.cuh"
 
